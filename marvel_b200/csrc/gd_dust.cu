@@ -1,13 +1,15 @@
 // gd_dust.cu -- DBdust's low-complexity scan (db/DBdust.c:219-487) on the device.
 //
 // The scan of one read is a sequential state machine (a window of triplet counts, a
-// left-trimmed run with its own counts, a short list of candidate intervals), so the GPU
-// runs one read per thread: a block of a few thousand to tens of thousands of reads keeps
-// the SMs busy, the counts and candidate list live in the thread's local memory (L1), and
-// each read's mask is written to its own slice of a device buffer.  Arithmetic follows the
+// left-trimmed run with its own counts, a short list of candidate intervals).  Its state
+// after position j follows from the last 2W bases alone, so k_dust_chunks cuts every read into
+// chunks and gives each a thread that starts 2W positions early (below).  With -b the sums are
+// doubles whose rounding carries the read's whole past, so k_dust_read scans one read per
+// thread.  Each read's mask is written to its own slice of a device buffer.  Arithmetic follows the
 // reference's types: integer pair-count sums, doubles for the thresholds, and with -b
 // (biased) double sums of count * skew, computed with explicit round-to-nearest operations
 // so that no multiply-add is fused (the reference's x86-64 build has none either).
+#include <climits>
 #include <cmath>
 
 #include "gd_dust.cuh"
@@ -42,10 +44,10 @@ __device__ __forceinline__ void dust_retire(int* mask, int& mtop, int beg, int e
     }
 }
 
-template <bool BIASED>
-__global__ void __launch_bounds__(64) k_dust(DevBlock blk, int W, double T, int thr2i, double thr2r,
-                                             const double* __restrict__ skew, int minlen, int* out,
-                                             int* __restrict__ nout)
+// -b: one read per thread, counts and candidates in local memory
+__global__ void __launch_bounds__(64) k_dust_read(DevBlock blk, int W, double T, double thr2r,
+                                                  const double* __restrict__ skew, int minlen, int* out,
+                                                  int* __restrict__ nout)
 {
     const int r = blockIdx.x * 64 + threadIdx.x;
     if (r >= blk.nreads)
@@ -67,21 +69,14 @@ __global__ void __launch_bounds__(64) k_dust(DevBlock blk, int W, double T, int 
         for (int i = 1; i <= W; i++)
             cd[i].next = (i < W) ? i + 1 : -1;
         int freel = 1, wb = -1, lb = -1;
-        long long wsi = 0, lsi = 0;
         double wsr = 0., lsr = 0.;
-        auto add = [&](int* cnt, int e, long long& si, double& sr) {
-            if (BIASED)
-                sr = __dadd_rn(sr, __dmul_rn((double)cnt[e], skew[e]));
-            else
-                si += cnt[e];
+        auto add = [&](int* cnt, int e, double& sr) {
+            sr = __dadd_rn(sr, __dmul_rn((double)cnt[e], skew[e]));
             cnt[e]++;
         };
-        auto del = [&](int* cnt, int e, long long& si, double& sr) {
+        auto del = [&](int* cnt, int e, double& sr) {
             cnt[e]--;
-            if (BIASED)
-                sr = __dsub_rn(sr, __dmul_rn((double)cnt[e], skew[e]));
-            else
-                si -= cnt[e];
+            sr = __dsub_rn(sr, __dmul_rn((double)cnt[e], skew[e]));
         };
         for (int j = 0; j < len; j++)
         {
@@ -90,33 +85,22 @@ __global__ void __launch_bounds__(64) k_dust(DevBlock blk, int W, double T, int 
             if (j > W - 3)
             {
                 d = dtrip(b, ++wb);
-                del(wcount, d, wsi, wsr);
+                del(wcount, d, wsr);
             }
-            add(wcount, c, wsi, wsr);
+            add(wcount, c, wsr);
             if (lb < wb)
             {
                 d = dtrip(b, ++lb);
-                del(lcount, d, lsi, lsr);
+                del(lcount, d, lsr);
             }
-            bool cut;
-            if (BIASED)
-            {
-                const double tr = __dmul_rn((double)lcount[c], skew[c]);
-                lcount[c]++;
-                lsr = __dadd_rn(lsr, tr);
-                cut = tr >= thr2r;
-            }
-            else
-            {
-                const int tr = lcount[c]++;
-                lsi += tr;
-                cut = tr >= thr2i;
-            }
-            if (cut)
+            const double tr = __dmul_rn((double)lcount[c], skew[c]);
+            lcount[c]++;
+            lsr = __dadd_rn(lsr, tr);
+            if (tr >= thr2r)
                 while (lb < j)
                 {
                     d = dtrip(b, ++lb);
-                    del(lcount, d, lsi, lsr);
+                    del(lcount, d, lsr);
                     if (d == c)
                         break;
                 }
@@ -131,17 +115,16 @@ __global__ void __launch_bounds__(64) k_dust(DevBlock blk, int W, double T, int 
                 cd[t].next = freel;
                 freel = t;
             }
-            double lsq = BIASED ? lsr : (double)lsi;
-            const double wsq = BIASED ? wsr : (double)wsi;
-            if (wsq <= __dmul_rn(lsq, T))
+            double lsq = lsr;
+            if (wsr <= __dmul_rn(lsq, T))
                 continue;
             int jp = cd[0].next, lp = 0, x;
             double ms = 0.;
             for (x = lb; x > wb; x--)
             {
                 d = dtrip(b, x);
-                add(lcount, d, lsi, lsr);
-                lsq = BIASED ? lsr : (double)lsi;
+                add(lcount, d, lsr);
+                lsq = lsr;
                 if (lsq >= __dmul_rn(T, (double)(j - x)))
                 {
                     for (; cd[jp].beg >= x; lp = jp, jp = cd[jp].next)
@@ -179,7 +162,7 @@ __global__ void __launch_bounds__(64) k_dust(DevBlock blk, int W, double T, int 
             for (x++; x <= lb; x++)
             {
                 d = dtrip(b, x);
-                del(lcount, d, lsi, lsr);
+                del(lcount, d, lsr);
             }
         }
         int t;
@@ -201,6 +184,238 @@ __global__ void __launch_bounds__(64) k_dust(DevBlock blk, int W, double T, int 
             mask[n++] = en;
         }
     nout[r] = n;
+}
+
+constexpr int DUST_CHUNK = 1024;  // interval starts per chunk
+constexpr int DT = 128;           // chunks per block
+
+// Without -b: a chunk of a read per thread.  A chunk owns the intervals that start in its
+// DUST_CHUNK positions.  The window (wb, j] and the run (lb, j] at position j follow from the
+// last W bases: wb = j - (W - 2), and lb is the least position at or beyond wb from which no
+// triplet is more frequent than the threshold allows (each step moves it just far enough).  A
+// candidate that starts at x is made, raised and tested at positions from x to x + W - 2 only, with
+// windows that reach back to x - W, against candidates that start at or behind x.  So a scan
+// begun 2W positions before the chunk has, from the chunk's first retirement on, exactly the
+// candidates of the whole read's scan.  The chunk's retired candidates come in order of their
+// starts and are merged as the reference merges them; k_dust_merge joins the chunks' lists,
+// which merges the same sequence in pieces.
+//
+// Bound by latency of the dependent steps, so the split is for warps in flight: one thread per
+// read (a 105 Mbp block of 10,020 reads) took 91 ms, its longest reads deciding; chunks give
+// 103,000 threads, 19 % of their steps spent on the starts.  Both counts of a triplet share
+// one shared-memory word ([triplet][thread], free of bank conflicts): the window's in the low
+// half, the run's in the high half.
+__global__ void __launch_bounds__(DT) k_dust_chunks(DevBlock blk, int W, double T, int thr2,
+                                                    const uint32_t* __restrict__ cfirst, unsigned nchunks, int* out,
+                                                    int* __restrict__ ccount)
+{
+    __shared__ unsigned cnt[64][DT];
+    const unsigned g = blockIdx.x * DT + threadIdx.x;
+    if (g >= nchunks)
+        return;
+    int lo = 0, hi = blk.nreads - 1;  // the read of this chunk: the last with cfirst <= g
+    while (lo < hi)
+    {
+        const int mid = (lo + hi + 1) >> 1;
+        if (cfirst[mid] <= g)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const int r = lo;
+    const int len = blk.rlen[r] - 2;
+    const uint8_t* b = blk.bases + blk.boff[r];
+    const int b0 = (int)(g - cfirst[r]) * DUST_CHUNK, b1 = min(b0 + DUST_CHUNK, len);
+    int* const list = out + blk.boff[r] + 4ll * r + b0;  // [begin, end] pairs, more than 3 apart
+    const int js = max(0, b0 - 2 * W), je = min(len, b1 + W - 2);
+    unsigned* const my = &cnt[0][threadIdx.x];
+    for (int e = 0; e < 64; e++)
+        my[e * DT] = 0;
+    DustCand cd[DUST_MAXW + 1];
+    cd[0].beg = -2;
+    cd[0].prev = cd[0].next = 0;
+    for (int i = 1; i <= W; i++)
+        cd[i].next = (i < W) ? i + 1 : -1;
+    int freel = 1, wb = js - 1, lb = js - 1, ws = 0, ls = 0;
+    int n = 0, mbeg = -2, mend = -2;  // the list and its open interval
+    auto retire = [&](int beg, int end) {
+        if (beg < b0 || beg >= b1)
+            return;  // another chunk's
+        const int c = end + 2;
+        if (mend + 1 >= beg)
+            mend = max(mend, c);
+        else
+        {
+            if (mbeg >= 0)
+            {
+                list[n++] = mbeg;
+                list[n++] = mend;
+            }
+            mbeg = beg;
+            mend = c;
+        }
+    };
+    // the triplets entering and leaving roll with their positions
+    int cj = (b[js] << 2) | b[js + 1], cw = cj, cl = cj;
+    int oldest = INT_MAX;  // start of the oldest candidate
+    bool full = false;
+    for (int j = js; j < je; j++)
+    {
+        cj = ((cj << 2) | b[j + 2]) & 63;
+        const int c = cj;
+        if (j - js > W - 3)
+        {
+            wb++;
+            cw = ((cw << 2) | b[wb + 2]) & 63;
+            const unsigned v = my[cw * DT] - 1u;
+            my[cw * DT] = v;
+            ws -= (int)(v & 0xffffu);
+        }
+        if (lb < wb)
+        {
+            lb++;
+            cl = ((cl << 2) | b[lb + 2]) & 63;
+            const unsigned v = my[cl * DT] - 0x10000u;
+            my[cl * DT] = v;
+            ls -= (int)(v >> 16);
+        }
+        {
+            const unsigned v = my[c * DT];
+            ws += (int)(v & 0xffffu);
+            const int tr = (int)(v >> 16);
+            ls += tr;
+            my[c * DT] = v + 0x10001u;
+            if (tr >= thr2)
+                while (lb < j)
+                {
+                    lb++;
+                    cl = ((cl << 2) | b[lb + 2]) & 63;
+                    const unsigned u = my[cl * DT] - 0x10000u;
+                    my[cl * DT] = u;
+                    ls -= (int)(u >> 16);
+                    if (cl == c)
+                        break;
+                }
+        }
+        // retire the oldest candidate once its start has left the window
+        if (oldest <= wb)
+        {
+            const int t = cd[0].prev;
+            retire(cd[t].beg, cd[t].end);
+            const int q = cd[t].prev;
+            cd[0].prev = q;
+            cd[q].next = 0;
+            cd[t].next = freel;
+            freel = t;
+            oldest = q ? cd[q].beg : INT_MAX;
+        }
+        double lsq = (double)ls;
+        if ((double)ws <= __dmul_rn(lsq, T))
+            continue;
+        int jp = cd[0].next, lp = 0, x;
+        double ms = 0.;
+        for (x = lb; x > wb; x--)
+        {
+            const int d = dtrip(b, x);
+            const unsigned v = my[d * DT];
+            ls += (int)(v >> 16);
+            my[d * DT] = v + 0x10000u;
+            lsq = (double)ls;
+            if (lsq >= __dmul_rn(T, (double)(j - x)))
+            {
+                for (; cd[jp].beg >= x; lp = jp, jp = cd[jp].next)
+                    if (cd[jp].score > ms)
+                        ms = cd[jp].score;
+                if (lsq >= __dmul_rn(ms, (double)(j - x)))
+                {
+                    ms = __ddiv_rn(lsq, (double)(j - x));
+                    if (cd[lp].beg == x)
+                    {
+                        cd[lp].end = j;
+                        cd[lp].score = ms;
+                    }
+                    else
+                    {
+                        const int q = freel;
+                        if (q < 0)
+                        {
+                            full = true;  // candidate pool exhausted
+                            break;
+                        }
+                        freel = cd[q].next;
+                        cd[q].beg = x;
+                        cd[q].end = j;
+                        cd[q].score = ms;
+                        cd[q].prev = lp;
+                        cd[lp].next = q;
+                        cd[q].next = jp;
+                        cd[jp].prev = q;
+                        if (jp == 0)
+                            oldest = x;
+                        lp = q;
+                    }
+                }
+            }
+        }
+        if (full)
+            break;
+        for (x++; x <= lb; x++)
+        {
+            const int d = dtrip(b, x);
+            const unsigned v = my[d * DT] - 0x10000u;
+            my[d * DT] = v;
+            ls -= (int)(v >> 16);
+        }
+    }
+    for (int t = cd[0].prev; t != 0 && !full; t = cd[t].prev)
+        retire(cd[t].beg, cd[t].end);
+    if (mbeg >= 0)
+    {
+        list[n++] = mbeg;
+        list[n++] = mend;
+    }
+    ccount[g] = full ? -1 : n;
+}
+
+// A read's chunk lists joined in place: intervals that touch merged, those of more than minlen
+// positions kept as [beg, end + 1)
+__global__ void __launch_bounds__(DT) k_dust_merge(DevBlock blk, const uint32_t* __restrict__ cfirst,
+                                                   const int* __restrict__ ccount, int minlen, int* out,
+                                                   int* __restrict__ nout)
+{
+    const int r = blockIdx.x * DT + threadIdx.x;
+    if (r >= blk.nreads)
+        return;
+    int* const mask = out + blk.boff[r] + 4ll * r;
+    int n = 0, beg = -2, end = -2;
+    bool full = false;
+    auto keep = [&]() {
+        if (beg >= 0 && end - beg >= minlen)
+        {
+            mask[n++] = beg;
+            mask[n++] = end + 1;
+        }
+    };
+    for (unsigned g = cfirst[r]; g < cfirst[r + 1]; g++)
+    {
+        const int* list = mask + (int)(g - cfirst[r]) * DUST_CHUNK;
+        const int m = ccount[g];
+        full |= m < 0;
+        for (int k = 0; k < m; k += 2)
+        {
+            const int lb = list[k], le = list[k + 1];
+            if (end + 1 >= lb)
+                end = max(end, le);
+            else
+            {
+                keep();
+                beg = lb;
+                end = le;
+            }
+        }
+    }
+    keep();
+    nout[r] = full ? -1 : n;
 }
 
 // packs read r's nout[r] ints to dst + off[r] (one warp per read)
@@ -227,8 +442,20 @@ int launch_dust_gather(const DevBlock& blk, const int* out, const int* nout, con
     return 0;
 }
 
-int launch_dust(const DevBlock& blk, int window, double thresh, int minlen, bool biased, const double* skew, int* out,
-                int* nout, cudaStream_t s)
+unsigned dust_chunks(const int32_t* rlen, int nreads, uint32_t* cfirst)
+{
+    unsigned n = 0;
+    for (int r = 0; r < nreads; r++)
+    {
+        cfirst[r] = n;
+        n += rlen[r] > 2 ? (unsigned)((rlen[r] - 2 + DUST_CHUNK - 1) / DUST_CHUNK) : 0u;
+    }
+    cfirst[nreads] = n;
+    return n;
+}
+
+int launch_dust(const DevBlock& blk, int window, double thresh, int minlen, bool biased, const double* skew,
+                const uint32_t* cfirst, unsigned nchunks, int* ccount, int* out, int* nout, cudaStream_t s)
 {
     if (blk.nreads <= 0)
         return 0;
@@ -237,13 +464,17 @@ int launch_dust(const DevBlock& blk, int window, double thresh, int minlen, bool
         gd_set_error("DUST window %d outside [3, %d]", window, DUST_MAXW);
         return -1;
     }
-    const int thr2i = (int)std::ceil(2. * thresh);
-    const double thr2r = 2. * thresh;
-    const unsigned grid = (unsigned)((blk.nreads + 63) / 64);
     if (biased)
-        k_dust<true><<<grid, 64, 0, s>>>(blk, window, thresh, thr2i, thr2r, skew, minlen, out, nout);
+        k_dust_read<<<(unsigned)((blk.nreads + 63) / 64), 64, 0, s>>>(blk, window, thresh, 2. * thresh, skew, minlen, out,
+                                                                     nout);
     else
-        k_dust<false><<<grid, 64, 0, s>>>(blk, window, thresh, thr2i, thr2r, skew, minlen, out, nout);
+    {
+        if (nchunks)
+            k_dust_chunks<<<(nchunks + DT - 1) / DT, DT, 0, s>>>(blk, window, thresh, (int)std::ceil(2. * thresh),
+                                                                 cfirst, nchunks, out, ccount);
+        k_dust_merge<<<(unsigned)((blk.nreads + DT - 1) / DT), DT, 0, s>>>(blk, cfirst, ccount, minlen, out, nout);
+        GD_LAUNCHED(1);
+    }
     GD_LAUNCHED(1);
     GD_CUDA(cudaGetLastError());
     return 0;

@@ -2082,13 +2082,19 @@ int64_t gd_dust(gd_context* c, int slot, int window, double thresh, int mflag, i
     GD_CUDA(cudaMemcpyAsync(&boff_end, S.blk.boff + n, 8, cudaMemcpyDeviceToHost, s));
     GD_CUDA(cudaStreamSynchronize(s));
     const size_t outints = (size_t)boff_end + 4ull * n + 8;
-    // scratch: per-read slices (k0), counts (flags), offsets (hoff), packed data (k1), weights (misc)
+    // the scan's chunks (not with -b, which scans whole reads)
+    std::vector<uint32_t> cfirst(n + 1);
+    const unsigned nchunks = biased ? 0 : dust_chunks(S.hrlen.data(), n, cfirst.data());
+    // scratch: per-read slices (k0), counts (flags), offsets (hoff), packed data (k1), weights (misc),
+    // first chunks (excl), counts per chunk (cnt)
     if (ensure(c->k0, outints * 4) || ensure(c->flags, (size_t)n * 4 + 4) || ensure(c->hoff, (size_t)n * 8 + 8) ||
-        ensure(c->misc, 1024))
+        ensure(c->misc, 1024) || ensure(c->excl, (size_t)n * 4 + 4) || ensure(c->cnt, (size_t)nchunks * 4 + 4))
         return -1;
     GD_CUDA(cudaMemcpyAsync(c->misc.p, skew, sizeof skew, cudaMemcpyHostToDevice, s));
-    if (launch_dust(S.blk, window, thresh, mflag - 1, biased != 0, P<double>(c->misc), P<int>(c->k0),
-                    P<int>(c->flags), s))
+    if (!biased)
+        GD_CUDA(cudaMemcpyAsync(c->excl.p, cfirst.data(), (size_t)(n + 1) * 4, cudaMemcpyHostToDevice, s));
+    if (launch_dust(S.blk, window, thresh, mflag - 1, biased != 0, P<double>(c->misc), P<uint32_t>(c->excl), nchunks,
+                    P<int>(c->cnt), P<int>(c->k0), P<int>(c->flags), s))
         return -1;
     std::vector<int> cnt(n);
     GD_CUDA(cudaMemcpyAsync(cnt.data(), c->flags.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
