@@ -204,6 +204,7 @@ struct gd_context
     bool srt_valid = false;
     HostBuf h_rec, h_tr;  // pinned staging for file writes
     DevBuf las_raw, las_off, las_rec, las_out;  // gd_las_sort
+    DevBuf vf_rec, vf_first, vf_trace, vf_seg, vf_list, vf_diff, vf_misc, vf_scr;  // gd_compute_trace_pts
     gd_stats stats;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, tev0 = nullptr, tev1 = nullptr;
     // learned triage: model (on), per-group feature/outcome collection (collect)
@@ -1437,7 +1438,8 @@ void gd_destroy(gd_context* c)
                       &c->tri_gstat, &c->tri_misc, &c->tri_x, &c->tri_y, &c->tri_perm, &c->tri_grad, &c->tri_m,
                       &c->tri_v, &c->tri_loss, &c->tri_w, &c->acc_rec, &c->acc_tr, &c->srt_rec, &c->srt_tr,
                       &c->okey0, &c->okey1, &c->oval0, &c->oval1, &c->olen, &c->las_raw, &c->las_off,
-                      &c->las_rec, &c->las_out, &c->ascr_w, &c->wide, &c->ascr_d};
+                      &c->las_rec, &c->las_out, &c->ascr_w, &c->wide, &c->ascr_d, &c->vf_rec, &c->vf_first,
+                      &c->vf_trace, &c->vf_seg, &c->vf_list, &c->vf_diff, &c->vf_misc, &c->vf_scr};
     for (DevBuf* b : bufs)
         release(*b);
     for (HostBuf* h : {&c->h_rec, &c->h_tr})
@@ -2256,9 +2258,11 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
     Slot& Cc = c->slot[cslot];
     const int TS = c->tspace;
     const int tbytes = TS <= 125 ? 1 : 2;
+    // the records' checks, their segments' places and the extent of their trace bytes
     bool any_comp = false;
-    std::vector<Segment> seg;
-    int R = 8;
+    std::vector<int64_t> first(n + 1);
+    int64_t nseg = 0;
+    uint64_t tlo = UINT64_MAX, thi = 0;
     for (int64_t r = 0; r < n; r++)
     {
         const gd_overlap& o = recs[r];
@@ -2274,70 +2278,67 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
             gd_set_error("gd_compute_trace_pts: record %lld has positions outside its reads", (long long)r);
             return -1;
         }
-        int comp = o.flags & 1;
-        any_comp |= comp != 0;
-        const uint8_t* t = trace + o.toff;
-        auto pt = [&](int i) { return tbytes == 1 ? (int)t[i] : (int)(t[2 * i] | (t[2 * i + 1] << 8)); };
-        // segments between consecutive trace points (align.c:5355-5389)
-        int ab = o.abpos, ae = (o.abpos / TS) * TS, bb = o.bbpos, be;
-        for (int i = 1; i < o.tlen - 2; i += 2)
+        any_comp |= (o.flags & 1) != 0;
+        const int inner = trace_inner(o.tlen);
+        first[r] = nseg;
+        nseg += inner + 1;
+        if (inner)
         {
-            ae += TS;
-            be = bb + pt(i);
-            seg.push_back(Segment{ar, br, ab, ae, bb, be, (int32_t)r, comp});
-            R = std::max(R, (ae - ab) + (be - bb) + 8);
-            ab = ae;
-            bb = be;
+            tlo = std::min(tlo, o.toff);
+            thi = std::max(thi, o.toff + (uint64_t)2 * inner * tbytes);
         }
-        seg.push_back(Segment{ar, br, ab, o.aepos, bb, o.bepos, (int32_t)r, comp});
-        R = std::max(R, (o.aepos - ab) + (o.bepos - bb) + 8);
     }
+    first[n] = nseg;
     if (any_comp && !Cc.loaded)
     {
         gd_set_error("gd_compute_trace_pts: complemented records need the complemented block in slot %d", cslot);
         return -1;
     }
-    int64_t nseg = (int64_t)seg.size();
-    int64_t nthreads = std::min<int64_t>(nseg, 148 * 512);
-    nthreads = (nthreads + 127) / 128 * 128;
-    DevBuf dseg, dscr, ddiff, dst;
-    int rc = -1;
-    do
+    if (thi <= tlo)
+        tlo = thi = 0;
+    const DevBlock& Cb = Cc.loaded ? Cc.blk : B.blk;
+    cudaStream_t s = c->s;
+    if (ensure(c->vf_rec, (size_t)n * sizeof(OutRec)) || ensure(c->vf_first, (size_t)(n + 1) * 8) ||
+        ensure(c->vf_trace, (size_t)(thi - tlo) + 16) || ensure(c->vf_seg, (size_t)nseg * sizeof(Segment)) ||
+        ensure(c->vf_list, (size_t)nseg * 4) || ensure(c->vf_diff, (size_t)n * 4) || ensure(c->vf_misc, 64))
+        return -1;
+    unsigned* misc = P<unsigned>(c->vf_misc);  // [0] segments for the general kernel, [1] R, [4..] status
+    DevStatus* dst = (DevStatus*)(misc + 4);
+    // all on the context's stream, which the kernels run on: a plain cudaMemcpy/cudaMemset goes
+    // to the legacy stream, which a non-blocking stream does not wait for
+    GD_CUDA(cudaMemcpyAsync(c->vf_rec.p, recs, (size_t)n * sizeof(OutRec), cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemcpyAsync(c->vf_first.p, first.data(), (size_t)(n + 1) * 8, cudaMemcpyHostToDevice, s));
+    if (thi > tlo)
+        GD_CUDA(cudaMemcpyAsync(c->vf_trace.p, trace + tlo, (size_t)(thi - tlo), cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemsetAsync(c->vf_diff.p, 0, (size_t)n * 4, s));
+    GD_CUDA(cudaMemsetAsync(c->vf_misc.p, 0, 64, s));
+    if (launch_trace_segments(P<OutRec>(c->vf_rec), n, P<int64_t>(c->vf_first), P<uint8_t>(c->vf_trace), tlo, TS, tbytes,
+                              A.blk.ufirst, B.blk.ufirst, P<Segment>(c->vf_seg), misc + 1, dst, s) ||
+        launch_trace_pts(A.blk, B.blk, Cb, P<Segment>(c->vf_seg), nseg, P<int>(c->vf_diff), P<unsigned>(c->vf_list), misc,
+                         s))
+        return -1;
+    unsigned h[8];
+    GD_CUDA(cudaMemcpyAsync(h, misc, sizeof h, cudaMemcpyDeviceToHost, s));
+    GD_CUDA(cudaStreamSynchronize(s));
+    if (h[0] && !h[4])
     {
-        if (ensure(dseg, nseg * sizeof(Segment)) || ensure(dscr, (size_t)nthreads * 3 * (2 * R + 1) * 4) ||
-            ensure(ddiff, n * 4) || ensure(dst, sizeof(DevStatus)))
-            break;
-        // all on the context's stream, which the kernel runs on: a plain cudaMemcpy/cudaMemset
-        // goes to the legacy stream, which a non-blocking stream does not wait for
-        if (cudaMemcpyAsync(dseg.p, seg.data(), nseg * sizeof(Segment), cudaMemcpyHostToDevice, c->s) != cudaSuccess ||
-            cudaMemsetAsync(ddiff.p, 0, n * 4, c->s) != cudaSuccess ||
-            cudaMemsetAsync(dst.p, 0, sizeof(DevStatus), c->s) != cudaSuccess)
-        {
-            gd_set_error("gd_compute_trace_pts: copies failed");
-            break;
-        }
-        if (launch_trace_pts(A.blk, B.blk, Cc.loaded ? Cc.blk : B.blk, P<Segment>(dseg), nseg, P<int>(dscr), R,
-                             (int)nthreads, P<int>(ddiff), P<DevStatus>(dst), c->s))
-            break;
-        DevStatus st;
-        if (cudaStreamSynchronize(c->s) != cudaSuccess ||
-            cudaMemcpy(&st, dst.p, sizeof st, cudaMemcpyDeviceToHost) != cudaSuccess ||
-            cudaMemcpy(diffs_out, ddiff.p, n * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
-        {
-            gd_set_error("gd_compute_trace_pts: %s", cudaGetErrorString(cudaGetLastError()));
-            break;
-        }
-        if (st.code)
-        {
-            gd_set_error("gd_compute_trace_pts: record %d failed (code %d)", st.where, st.code);
-            break;
-        }
-        rc = 0;
-    } while (0);
-    DevBuf* all[] = {&dseg, &dscr, &ddiff, &dst};
-    for (DevBuf* b : all)
-        release(*b);
-    return rc;
+        // segments too long or too different for the fast kernel's bands
+        const int R = (int)h[1];
+        const int64_t nthreads = (std::min<int64_t>(h[0], 148 * 512) + 127) / 128 * 128;
+        if (ensure(c->vf_scr, (size_t)nthreads * 3 * (2 * (size_t)R + 1) * 4) ||
+            launch_trace_pts_list(A.blk, B.blk, Cb, P<Segment>(c->vf_seg), P<unsigned>(c->vf_list), h[0],
+                                  P<int>(c->vf_scr), R, (int)nthreads, P<int>(c->vf_diff), dst, s))
+            return -1;
+        GD_CUDA(cudaMemcpyAsync(h, misc, sizeof h, cudaMemcpyDeviceToHost, s));
+    }
+    GD_CUDA(cudaMemcpyAsync(diffs_out, c->vf_diff.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
+    GD_CUDA(cudaStreamSynchronize(s));
+    if (h[4])
+    {
+        gd_set_error("gd_compute_trace_pts: record %d failed (code %d)", (int)h[5], (int)h[4]);
+        return -1;
+    }
+    return 0;
 }
 
 int gd_reset_overlap_buffer(gd_context* c)
