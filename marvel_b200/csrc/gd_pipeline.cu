@@ -977,7 +977,7 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
     const int seed_test = c->variant == 1 ? c->hitmin : 0;
     if (launch_select_groups(P<uint32_t>(c->starts), nst, nhits, minhit, hkey, hdiag, c->binshift, c->kmer, seed_test,
                              hb, P<int32_t>(A.rlen), P<int32_t>(B.rlen), P<uint2>(c->groups), P<uint32_t>(c->gcost),
-                             P<uint32_t>(c->gidx), d_ng, s))
+                             P<uint32_t>(c->gidx), d_ng, c->sched_edges.empty(), s))
         return -1;
     unsigned ng = 0;
     GD_CUDA(cudaMemcpyAsync(&ng, d_ng, 4, cudaMemcpyDeviceToHost, s));
