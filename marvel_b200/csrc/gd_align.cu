@@ -3627,8 +3627,10 @@ int launch_align_pairs(const DevBlock& A, const DevBlock& B, const uint64_t* hke
 // Local_Alignment batch (tests)
 // ------------------------------------------------------------------------------------------
 
+// PK: the sequences' 2-bit copies apk / bpk, byte 0 of the buffers at index apk0 / bpk0
+template <bool PK>
 __global__ void __launch_bounds__(ALIGN_WARPS * 32)
-    k_la_batch(const uint8_t* abase, const int64_t* aoff, const int32_t* alen, const uint8_t* bbase,
+    k_la_batch(const uint32_t* apk, uint32_t apk0, const uint32_t* bpk, uint32_t bpk0, const uint8_t* abase, const int64_t* aoff, const int32_t* alen, const uint8_t* bbase,
                const int64_t* boff, const int32_t* blen, const int32_t* diag, const int32_t* anti, int nseeds,
                AlignParams P, AlignScratch sc, int32_t* out12, uint16_t* tr, int trstride, int64_t* cells,
                DevStatus* st)
@@ -3654,8 +3656,8 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32)
         w.item = sd;
         const uint8_t* aseq = abase + aoff[sd];
         const uint8_t* bseq = bbase + boff[sd];
-        local_alignment<RING, false>(w, P, aseq, bseq, nullptr, 0, nullptr, 0, alen[sd], blen[sd], P.comp, diag[sd],
-                                     anti[sd]);
+        local_alignment<RING, PK>(w, P, aseq, bseq, apk, apk0 + (uint32_t)aoff[sd], bpk, bpk0 + (uint32_t)boff[sd],
+                                  alen[sd], blen[sd], P.comp, diag[sd], anti[sd]);
         if (w.err)
         {
             if (w.err == 2 && lane == 0)
@@ -3701,13 +3703,20 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32)
 int launch_la_batch(const uint8_t* aseq_base, const int64_t* aoff, const int32_t* alen, const uint8_t* bseq_base,
                     const int64_t* boff, const int32_t* blen, const int32_t* diag, const int32_t* anti, int nseeds,
                     AlignParams p, AlignScratch sc, int32_t* out12, uint16_t* tr, int trstride, int64_t* cells,
-                    DevStatus* st, cudaStream_t s)
+                    DevStatus* st, cudaStream_t s, const uint32_t* apk, uint32_t apk0, const uint32_t* bpk,
+                    uint32_t bpk0)
 {
     if (nseeds <= 0)
         return 0;
     int grid = gd_cdiv(sc.nwarps, ALIGN_WARPS);
-    k_la_batch<<<grid, ALIGN_WARPS * 32, 0, s>>>(aseq_base, aoff, alen, bseq_base, boff, blen, diag, anti, nseeds, p, sc,
-                                                 out12, tr, trstride, cells, st);
+    if (apk)
+        k_la_batch<true><<<grid, ALIGN_WARPS * 32, 0, s>>>(apk, apk0, bpk, bpk0, aseq_base, aoff, alen, bseq_base, boff,
+                                                           blen, diag, anti, nseeds, p, sc, out12, tr, trstride, cells,
+                                                           st);
+    else
+        k_la_batch<false><<<grid, ALIGN_WARPS * 32, 0, s>>>(nullptr, 0, nullptr, 0, aseq_base, aoff, alen, bseq_base,
+                                                            boff, blen, diag, anti, nseeds, p, sc, out12, tr, trstride,
+                                                            cells, st);
     GD_LAUNCHED(1);
     GD_CUDA(cudaGetLastError());
     return 0;

@@ -204,6 +204,7 @@ struct gd_context
     bool srt_valid = false;
     HostBuf h_rec, h_tr;  // pinned staging for file writes
     DevBuf las_raw, las_off, las_rec, las_out;  // gd_las_sort
+    DevBuf lb_a, lb_b, lb_pka, lb_pkb, lb_in, lb_out, lb_tr;  // gd_local_alignment_batch
     DevBuf vf_rec, vf_first, vf_trace, vf_seg, vf_list, vf_diff, vf_misc, vf_scr;  // gd_compute_trace_pts
     gd_stats stats;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, tev0 = nullptr, tev1 = nullptr;
@@ -1439,7 +1440,8 @@ void gd_destroy(gd_context* c)
                       &c->tri_v, &c->tri_loss, &c->tri_w, &c->acc_rec, &c->acc_tr, &c->srt_rec, &c->srt_tr,
                       &c->okey0, &c->okey1, &c->oval0, &c->oval1, &c->olen, &c->las_raw, &c->las_off,
                       &c->las_rec, &c->las_out, &c->ascr_w, &c->wide, &c->ascr_d, &c->vf_rec, &c->vf_first,
-                      &c->vf_trace, &c->vf_seg, &c->vf_list, &c->vf_diff, &c->vf_misc, &c->vf_scr};
+                      &c->vf_trace, &c->vf_seg, &c->vf_list, &c->vf_diff, &c->vf_misc, &c->vf_scr, &c->lb_a, &c->lb_b,
+                      &c->lb_pka, &c->lb_pkb, &c->lb_in, &c->lb_out, &c->lb_tr};
     for (DevBuf* b : bufs)
         release(*b);
     for (HostBuf* h : {&c->h_rec, &c->h_tr})
@@ -2427,8 +2429,11 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     }
     if (nseeds <= 0)
         return 0;
-    DevBuf da, db, dao, dal, dbo, dbl, dd, dn, dout, dtr, dc, dst;
-    int rc = -1;
+    if (alen_total + 256 > 0xffffffffll || blen_total + 256 > 0xffffffffll)
+    {
+        gd_set_error("Local_Alignment batch: sequences beyond this build's 32-bit base index");
+        return -1;
+    }
     int maxlen = 0;
     for (int i = 0; i < nseeds; i++)
         maxlen = std::max(maxlen, std::max(alen[i], blen[i]));
@@ -2444,57 +2449,56 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     int grid = 0;
     if (align_grid(&grid))
         return -1;
-    int nwarps = std::min(grid * ALIGN_WARPS, ((nseeds + ALIGN_WARPS - 1) / ALIGN_WARPS) * ALIGN_WARPS);
-    int ptscap = 4 * (2 * (maxlen / c->tspace + 2)) + 32;
+    const int nwarps = std::min(grid * ALIGN_WARPS, ((nseeds + ALIGN_WARPS - 1) / ALIGN_WARPS) * ALIGN_WARPS);
+    const int ptscap = 4 * (2 * (maxlen / c->tspace + 2)) + 32;
     AlignScratch sc{};
-    DevBuf scr;
-    do
+    // the context keeps these buffers (the scratch is the pair aligner's); the call's own cudaMalloc
+    // and cudaFree of 2 GB took most of its time
+    const size_t n8 = (size_t)nseeds * 8, n4 = (size_t)nseeds * 4;
+    const int64_t wa = (alen_total + 128 + 15) / 16 + 1, wb = (blen_total + 128 + 15) / 16 + 1;
+    if (ensure(c->lb_a, alen_total + 128) || ensure(c->lb_b, blen_total + 128) || ensure(c->lb_pka, wa * 4) ||
+        ensure(c->lb_pkb, wb * 4) || ensure(c->lb_in, 2 * n8 + 4 * n4) || ensure(c->lb_out, n8 + 12 * n4 + 64) ||
+        ensure(c->lb_tr, (size_t)nseeds * trstride * 2) ||
+        ensure(c->ascr, align_scratch_bytes(nwarps, c->pcap, ptscap, 4, 4, 4)))
+        return -1;
+    align_scratch_carve(&sc, c->ascr.p, nwarps, c->pcap, ptscap, 4, 4, 4);
+    cudaStream_t s = c->s;
+    int64_t *d_ao = P<int64_t>(c->lb_in), *d_bo = d_ao + nseeds;
+    int32_t *d_al = (int32_t*)(d_bo + nseeds), *d_bl = d_al + nseeds, *d_dg = d_bl + nseeds, *d_an = d_dg + nseeds;
+    DevStatus* d_st = P<DevStatus>(c->lb_out);
+    int64_t* d_cells = (int64_t*)(P<char>(c->lb_out) + 64);
+    int32_t* d_out = (int32_t*)(d_cells + nseeds);
+    // sequences: caller buffers hold [4, read, 4, read, ...] with offsets relative to index 0
+    GD_CUDA(cudaMemsetAsync(c->lb_a.p, 4, alen_total + 128, s));
+    GD_CUDA(cudaMemsetAsync(c->lb_b.p, 4, blen_total + 128, s));
+    GD_CUDA(cudaMemcpyAsync(P<uint8_t>(c->lb_a) + 64, abases, alen_total, cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemcpyAsync(P<uint8_t>(c->lb_b) + 64, bbases, blen_total, cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemcpyAsync(d_ao, aoff, n8, cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemcpyAsync(d_bo, boff, n8, cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemcpyAsync(d_al, alen, n4, cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemcpyAsync(d_bl, blen, n4, cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemcpyAsync(d_dg, diag, n4, cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemcpyAsync(d_an, anti, n4, cudaMemcpyHostToDevice, s));
+    GD_CUDA(cudaMemsetAsync(c->lb_out.p, 0, n8 + 12 * n4 + 64, s));
+    if (launch_pack2(P<uint8_t>(c->lb_a), alen_total + 128, P<uint32_t>(c->lb_pka), wa, s) ||
+        launch_pack2(P<uint8_t>(c->lb_b), blen_total + 128, P<uint32_t>(c->lb_pkb), wb, s) ||
+        launch_la_batch(P<uint8_t>(c->lb_a) + 64, d_ao, d_al, P<uint8_t>(c->lb_b) + 64, d_bo, d_bl, d_dg, d_an, nseeds,
+                        ap, sc, d_out, P<uint16_t>(c->lb_tr), trstride, d_cells, d_st, s, P<uint32_t>(c->lb_pka), 64,
+                        P<uint32_t>(c->lb_pkb), 64))
+        return -1;
+    DevStatus st;
+    GD_CUDA(cudaMemcpyAsync(&st, d_st, sizeof st, cudaMemcpyDeviceToHost, s));
+    GD_CUDA(cudaStreamSynchronize(s));
+    if (st.code)
     {
-        if (ensure(da, alen_total + 128) || ensure(db, blen_total + 128) || ensure(dao, nseeds * 8) ||
-            ensure(dal, nseeds * 4) || ensure(dbo, nseeds * 8) || ensure(dbl, nseeds * 4) ||
-            ensure(dd, nseeds * 4) || ensure(dn, nseeds * 4) || ensure(dout, (size_t)nseeds * 48) ||
-            ensure(dtr, (size_t)nseeds * trstride * 2) || ensure(dc, nseeds * 8) || ensure(dst, sizeof(DevStatus)) ||
-            ensure(scr, align_scratch_bytes(nwarps, c->pcap, ptscap, 4, 4, 4)))
-            break;
-        align_scratch_carve(&sc, scr.p, nwarps, c->pcap, ptscap, 4, 4, 4);
-        // sequences: caller buffers hold [4, read, 4, read, ...] with offsets relative to index 0
-        if (cudaMemset(da.p, 4, alen_total + 128) != cudaSuccess || cudaMemset(db.p, 4, blen_total + 128) != cudaSuccess)
-            break;
-        cudaMemcpy((uint8_t*)da.p + 64, abases, alen_total, cudaMemcpyHostToDevice);
-        cudaMemcpy((uint8_t*)db.p + 64, bbases, blen_total, cudaMemcpyHostToDevice);
-        cudaMemcpy(dao.p, aoff, nseeds * 8, cudaMemcpyHostToDevice);
-        cudaMemcpy(dal.p, alen, nseeds * 4, cudaMemcpyHostToDevice);
-        cudaMemcpy(dbo.p, boff, nseeds * 8, cudaMemcpyHostToDevice);
-        cudaMemcpy(dbl.p, blen, nseeds * 4, cudaMemcpyHostToDevice);
-        cudaMemcpy(dd.p, diag, nseeds * 4, cudaMemcpyHostToDevice);
-        cudaMemcpy(dn.p, anti, nseeds * 4, cudaMemcpyHostToDevice);
-        cudaMemset(dst.p, 0, sizeof(DevStatus));
-        cudaMemset(dout.p, 0, (size_t)nseeds * 48);
-        if (launch_la_batch((const uint8_t*)da.p + 64, P<int64_t>(dao), P<int32_t>(dal), (const uint8_t*)db.p + 64,
-                            P<int64_t>(dbo), P<int32_t>(dbl), P<int32_t>(dd), P<int32_t>(dn), nseeds, ap, sc,
-                            P<int32_t>(dout), P<uint16_t>(dtr), trstride, P<int64_t>(dc), P<DevStatus>(dst), 0))
-            break;
-        if (cudaDeviceSynchronize() != cudaSuccess)
-        {
-            gd_set_error("Local_Alignment batch failed: %s", cudaGetErrorString(cudaGetLastError()));
-            break;
-        }
-        DevStatus st;
-        cudaMemcpy(&st, dst.p, sizeof st, cudaMemcpyDeviceToHost);
-        if (st.code)
-        {
-            gd_set_error("Local_Alignment batch: seed %d failed with code %d (info %d)", st.where, st.code, st.info);
-            break;
-        }
-        cudaMemcpy(out12, dout.p, (size_t)nseeds * 48, cudaMemcpyDeviceToHost);
-        cudaMemcpy(trace, dtr.p, (size_t)nseeds * trstride * 2, cudaMemcpyDeviceToHost);
-        cudaMemcpy(cells, dc.p, nseeds * 8, cudaMemcpyDeviceToHost);
-        rc = 0;
-    } while (0);
-    DevBuf* all[] = {&da, &db, &dao, &dal, &dbo, &dbl, &dd, &dn, &dout, &dtr, &dc, &dst, &scr};
-    for (DevBuf* b : all)
-        release(*b);
-    return rc;
+        gd_set_error("Local_Alignment batch: seed %d failed with code %d (info %d)", st.where, st.code, st.info);
+        return -1;
+    }
+    GD_CUDA(cudaMemcpyAsync(out12, d_out, 12 * n4, cudaMemcpyDeviceToHost, s));
+    GD_CUDA(cudaMemcpyAsync(trace, c->lb_tr.p, (size_t)nseeds * trstride * 2, cudaMemcpyDeviceToHost, s));
+    GD_CUDA(cudaMemcpyAsync(cells, d_cells, n8, cudaMemcpyDeviceToHost, s));
+    GD_CUDA(cudaStreamSynchronize(s));
+    return 0;
 }
 
 // ---------------------------------------------------------------------------------------
