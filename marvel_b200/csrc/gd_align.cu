@@ -10,8 +10,10 @@
 // is the reference's M), HA/HB (pebble heads), NA/NB (next trace-point marks) live in two
 // per-warp shared-memory rings indexed by diagonal, one per wave parity: each wave reads
 // the previous wave for diagonals k-1, k, k+1 and writes the other ring, which is the
-// reference's in-place update order.  The reference's sequential "c > besta" scan over
-// diagonals becomes a warp prefix-max in scan order; its clip bookkeeping becomes ballots.
+// reference's in-place update order.  A band of at most 30 diagonals (most waves) is held in
+// registers instead, a diagonal per lane, and updated by shuffles (wave_regs).  The reference's
+// sequential "c > besta" scan over diagonals becomes a warp prefix-max in scan order; its clip
+// bookkeeping becomes ballots.
 // Pebbles go to a per-warp global arena; the two trace-point chains are unwound by lane 0.
 // Match extension compares 4 bases per step with 32-bit XOR windows.
 //
@@ -89,6 +91,12 @@ struct ChunkEdge
     int v, ha, hb, na, nb, pad;
 };
 
+// The wave's state between waves (forward_wave / reverse_wave's loop-carried locals).
+struct WaveVars
+{
+    int hgh, low, dif, more, aclip, bclip, besta, lasta, npeb;
+};
+
 struct LAPath
 {
     int abpos, bbpos, aepos, bepos, diffs, tlen, toff, pad;
@@ -103,6 +111,9 @@ struct WarpSmem
     int trim[5];  // the trim point (anti-diagonal, y, diffs, A and B pebble heads), written by its lane
     int clipm[6];  // the clip fallback: M count, anti-diagonal, y, diffs, A and B pebble heads
     int besty;    // y of the best anti-diagonal
+    WaveVars wv;  // wave_ring's state, its error and cells
+    int wv_err;
+    unsigned wv_cells;
     ChunkEdge edge[ring_of<RG>() / 32 > 1 ? ring_of<RG>() / 32 - 1 : 1];  // [ch]: chunk ch's last diagonal
 };
 
@@ -322,12 +333,6 @@ __device__ __forceinline__ int peb_one(WarpCtx<RG>& w, int& npeb, int ptr, int d
         w.peb[idx] = make_int4(ptr, diag, diff, mark);
     return idx;
 }
-
-// The wave's state between waves (forward_wave / reverse_wave's loop-carried locals).
-struct WaveVars
-{
-    int hgh, low, dif, more, aclip, bclip, besta, lasta, npeb;
-};
 
 // forward_wave (FWD) / reverse_wave (!FWD) restated, with lanes over diagonals, in three
 // parts so that a caller can run it a wave at a time: wave_begin (the 0-wave from the seed
@@ -921,6 +926,321 @@ __device__ __forceinline__ bool wave_step(const bool FWD, WarpCtx<RG>& w, WaveVa
     w.cells += hgh - low + 1;
     wvars.hgh = hgh; wvars.low = low; wvars.dif = dif; wvars.more = more; wvars.aclip = aclip; wvars.bclip = bclip; wvars.besta = besta; wvars.lasta = lasta; wvars.npeb = npeb;
     return true;
+}
+
+// The waves of a narrow band with the wave vectors in registers: diagonal k lives in the lane
+// (FWD ? -k : k) & 31, so lanes in order are diagonals in scan order, the neighbours of a
+// diagonal are the neighbouring lanes, and a band that moves needs no copying.  Lanes outside
+// the band hold V = none, which stands for the reference's sentinels; a band of at most 30
+// diagonals keeps both of its ends beside such a lane.  Against wave_step (the ring form): the
+// predecessors' values come by six shuffles instead of eight shared-memory loads and six
+// stores, there is one chunk and no barrier, and the marks NA / NB are not kept at all: the next
+// mark of a path is the first boundary beyond its furthest point (V of a diagonal only grows,
+// and a new diagonal starts at or beyond its neighbour's point, so the marks the reference
+// carries per diagonal are never ahead of or behind that), which the predecessor's position
+// gives, and so no pebble is read back for its mark either.  On a 21 Mbp block (25 M waves per
+// orientation) the kernel issues 6.6 G warp instructions instead of 8.2 G and takes 7.9 ms
+// instead of 9.4; it stays bound by issue (76 % of the slots) and the dependent chain of a wave.
+//
+// Runs waves until the wave loop ends (false; or an error in w.err) or the band or anything
+// unusual asks for wave_step (true; the state is then in the ring).
+constexpr int REGS_BAND = 30;  // widest band held in registers
+constexpr int REGS_BACK = 24;  // a band this narrow returns to registers
+
+template <bool FWD, int RG>
+__device__ __forceinline__ bool wave_regs(WarpCtx<RG>& w, WaveVars& wvars, const AlignParams& P, const uint32_t* apk,
+                                          uint32_t ag, const uint32_t* bpk, uint32_t bg, int alen, int blen, int boff)
+{
+    WaveSmem<RG>& R = w.sm->ws;
+    const int lane = w.lane;
+    const int TS = P.tspace;
+    constexpr int S = FWD ? 1 : -1;
+    constexpr int VNONE = FWD ? -1 : INT_MAX;
+    const int PATH_AVE = P.ave_path;
+    int* const trim = w.sm->trim;
+    int* const clipm = w.sm->clipm;
+    int hgh = wvars.hgh, low = wvars.low, dif = wvars.dif, besta = wvars.besta, lasta = wvars.lasta, npeb = wvars.npeb;
+    int kbest = besta - 2 * w.sm->besty;  // the best point's diagonal
+    unsigned cells = 0;
+    auto divTS = [&](int n) { return (int)__umulhi((uint32_t)n, P.tsmagic); };
+    // the wave loop ends when the band no longer moves the last good point (or a read end was met)
+    constexpr int ENDED = FWD ? -(1 << 28) : 1 << 28;
+    auto ended = [&]() { return FWD ? lasta < besta - TRIM_MLAG : lasta > besta + TRIM_MLAG; };
+    if (!wvars.more)
+        lasta = ENDED;
+    // the band from the ring
+    int v = VNONE;
+    uint32_t t0 = 0, t1 = 0;
+    int ha = 0, hb = 0;
+    {
+        const int s0 = FWD ? -hgh : low;
+        const int p = (lane - s0) & 31;
+        if (low <= hgh && hgh - low < REGS_BAND && p <= hgh - low)
+        {
+            const int k = FWD ? hgh - p : low + p;
+            v = R.V[0][k & RM];
+            t0 = (uint32_t)R.T[0][k & RM];
+            t1 = (uint32_t)(R.T[0][k & RM] >> 32);
+            ha = R.HA[0][k & RM];
+            hb = R.HB[0][k & RM];
+        }
+    }
+    bool again = false;
+    while (!ended())
+    {
+        if ((unsigned)(hgh - low) > (unsigned)(REGS_BAND - 3) || dif >= alen + blen + 2)
+        {
+            again = true;  // too wide, or what wave_step reports as an error
+            break;
+        }
+        // widen the band by one each side (align.c:636-745)
+        low--;
+        hgh++;
+        dif++;
+        const int s0 = FWD ? -hgh : low;
+        const int p = (lane - s0) & 31;
+        bool valid = p <= hgh - low;
+        const int k = FWD ? -(s0 + p) : s0 + p;
+        // the furthest of the three predecessors (align.c:748-797)
+        const int vP = __shfl_sync(GD_FULL, v, lane - 1), vN = __shfl_sync(GD_FULL, v, lane + 1);
+        const bool nC = FWD ? v < vN : v > vN;
+        const bool pN = FWD ? vN < vP : vN > vP;
+        const bool pC = FWD ? v < vP : v > vP;
+        const bool useP = nC ? pN : pC;
+        const bool useN = nC && !pN;
+        const int src = lane + (useP ? -1 : (useN ? 1 : 0));
+        int c = (useP ? vP : (useN ? vN : v)) + ((useP || useN) ? S : 2 * S);
+        t0 = __shfl_sync(GD_FULL, t0, src);
+        t1 = __shfl_sync(GD_FULL, t1, src);
+        ha = __shfl_sync(GD_FULL, ha, src);
+        hb = __shfl_sync(GD_FULL, hb, src);
+        int y = (c - k) >> 1;
+        bool bend = false, aend = false, needA = false, needB = false;
+        int ma = 0, mb = 0, key = INT_MIN;
+        if (valid)
+        {
+            const int y0 = y, x0 = y + k;
+            y = snake_pk(FWD, apk, ag, bpk, bg, y, k, alen, blen, bend, aend);
+            const int L = FWD ? y - y0 : y0 - y;
+            if ((unsigned)L < 31u)
+            {
+                t1 = __funnelshift_l(t0, t1, L + 1);
+                t0 = (t0 << (L + 1)) | ((1u << L) - 1u);
+            }
+            else
+            {
+                unsigned long long b = (((unsigned long long)t1 << 32) | t0) << 1;
+                b = (L >= 61) ? ~0ull : ((b << L) | ((1ull << L) - 1ull));
+                t0 = (uint32_t)b;
+                t1 = (uint32_t)(b >> 32);
+            }
+            c = (y << 1) + k;
+            key = ((FWD ? c : -c) << 5) | (31 - p);
+            // the first marks beyond the predecessor, which stands at x0 - S or x0, y0 - S or y0
+            const int xp = useP ? x0 : x0 - S, yp = useN ? y0 : y0 - S;
+            if (FWD)
+            {
+                ma = (divTS(xp) + 1) * TS;
+                mb = divTS(yp + TS - boff) * TS + boff;
+                needA = y + k >= ma;
+                needB = y >= mb;
+            }
+            else
+            {
+                ma = (divTS(xp + TS - 1) - 1) * TS;
+                mb = (divTS(yp + TS - boff - 1) - 1) * TS + boff;
+                needA = y + k <= ma;
+                needB = y <= mb;
+            }
+        }
+        // trace points of A and B that the step crosses (align.c:826-878)
+        while (__any_sync(GD_FULL, needA || needB))
+        {
+            const unsigned mA = __ballot_sync(GD_FULL, needA), mB = __ballot_sync(GD_FULL, needB);
+            const int base = npeb;
+            npeb += __popc(mA) + __popc(mB);
+            if (npeb > w.pcap)
+            {
+                if (lane == 0)
+                    gd_fail(w.st, GD_ERR_PEBBLES, w.item, w.pcap);
+                w.err = 1;
+                return false;
+            }
+            if (needA)
+            {
+                const int idx = base + __popc(mA & lanemask_lt());
+                w.peb[idx] = make_int4(ha, k, dif, ma);
+                ha = idx;
+                ma += S * TS;
+                needA = FWD ? y + k >= ma : y + k <= ma;
+            }
+            if (needB)
+            {
+                const int idx = base + __popc(mA) + __popc(mB & lanemask_lt());
+                w.peb[idx] = make_int4(hb, k, dif, mb);
+                hb = idx;
+                mb += S * TS;
+                needB = FWD ? y >= mb : y <= mb;
+            }
+        }
+        // ballots in scan order: bit p of rot(m) is the diagonal p behind the band's first
+        auto rot = [&](unsigned m) { return __funnelshift_r(m, m, (unsigned)s0); };
+        const int hgh0 = hgh, low0 = low;
+        auto at = [&](int q) { return FWD ? hgh0 - q : low0 + q; };
+        // the best point (align.c:880-897): the first diagonal in scan order with the largest V,
+        // value and place in one reduction
+        const int wbest = FWD ? besta : -besta;
+        const bool q1 = (key >> 5) > wbest && __popc(t0) + __popc(t1 & (uint32_t)(MASK61 >> 32)) >= PATH_AVE;
+        const bool q2 = q1 && trim_ok(t0, P.table, P.score);
+        const int kmax = __reduce_max_sync(GD_FULL, key);
+        const bool better = (kmax >> 5) > wbest;
+        const int jm = 31 - (kmax & 31);
+        const unsigned m1 = __ballot_sync(GD_FULL, q1);
+        bool p1j = false;
+        if (better)
+        {
+            p1j = (m1 >> ((s0 + jm) & 31)) & 1;
+            besta = FWD ? kmax >> 5 : -(kmax >> 5);
+            kbest = at(jm);
+            if (p1j)
+                lasta = besta;
+        }
+        // read ends (align.c:798-824, 899-944)
+        if (__any_sync(GD_FULL, bend || aend))
+        {
+            const unsigned bm = rot(__ballot_sync(GD_FULL, bend));
+            const unsigned am = rot(__ballot_sync(GD_FULL, aend));
+            const int besty = (besta - kbest) >> 1;
+            const int M = __popc(t0) + __popc(t1 & (uint32_t)(MASK61 >> 32));
+            auto clip = [&](int q) {
+                if (p == q && clipm[0] <= M)
+                {
+                    clipm[0] = M;
+                    clipm[1] = c;
+                    clipm[2] = (c - k) / 2;
+                    clipm[3] = dif;
+                    clipm[4] = ha;
+                    clipm[5] = hb;
+                }
+                __syncwarp();
+            };
+            if (am)  // the last A end in scan order
+            {
+                const int q = 31 - __clz(am);
+                if (FWD)
+                    hgh = at(q) - 1;
+                else
+                    low = at(q) + 1;
+                clip(q);
+            }
+            if (bm)  // the first B end
+            {
+                const int q = __ffs(bm) - 1;
+                if (FWD ? low <= at(q) : hgh >= at(q))
+                {
+                    if (FWD)
+                        low = at(q) + 1;
+                    else
+                        hgh = at(q) - 1;
+                    clip(q);
+                }
+            }
+            valid = valid && k >= low && k <= hgh;
+            if (!(FWD ? (besty < blen && besta - besty < alen) : (besty > 0 && besta - besty > 0)))
+                wvars.more = 0;
+        }
+        // drop diagonals more than WAVE_LAG behind the best (align.c:946-955)
+        const unsigned gm =
+            rot(__ballot_sync(GD_FULL, valid && (FWD ? c >= besta - WAVE_LAG : c <= besta + WAVE_LAG)));
+        // the trim point: the maximum's when it passes both tests
+        const unsigned m2 = __ballot_sync(GD_FULL, q2);
+        if (better)
+        {
+            int jt = jm;
+            if (!((m2 >> ((s0 + jm) & 31)) & 1))
+            {
+                // a diagonal before the maximum can be a record that matters only when it passes
+                // the first test, and the second or where the maximum fails the first
+                jt = -1;
+                const unsigned before = (1u << jm) - 1u;
+                const unsigned mq1 = rot(m1) & before, mq2 = rot(m2) & before;
+                if (mq1 && (!p1j || mq2))
+                {
+                    int incl = key >> 5;
+                    for (int o = 1; o < jm; o <<= 1)
+                    {
+                        const int t = __shfl_sync(GD_FULL, incl, lane - o);
+                        if (p >= o)
+                            incl = max(incl, t);
+                    }
+                    int excl = __shfl_sync(GD_FULL, incl, lane - 1);
+                    if (p == 0)
+                        excl = INT_MIN;
+                    const unsigned mrec =
+                        rot(__ballot_sync(GD_FULL, p < jm && (key >> 5) > max(wbest, excl)));
+                    const unsigned r1 = mrec & mq1, r2 = mrec & mq2;
+                    if (r1 && !p1j)
+                        lasta = __shfl_sync(GD_FULL, c, s0 + 31 - __clz(r1));
+                    if (r2)
+                        jt = 31 - __clz(r2);
+                }
+            }
+            if (p == jt)
+            {
+                trim[0] = c;
+                trim[1] = y;
+                trim[2] = dif;
+                trim[3] = ha;
+                trim[4] = hb;
+            }
+            __syncwarp();  // a later wave's trim point overwrites these
+        }
+        if (!wvars.more)
+            lasta = ENDED;
+        v = VNONE;
+        if (gm == 0)
+        {
+            hgh = low - 1;
+            again = !ended();  // every diagonal fell behind: wave_step reports it
+            break;
+        }
+        const int qf = __ffs(gm) - 1, ql = 31 - __clz(gm);
+        hgh = FWD ? hgh0 - qf : low0 + ql;
+        low = FWD ? hgh0 - ql : low0 + qf;
+        cells += hgh - low + 1;
+        if ((unsigned)(p - qf) <= (unsigned)(ql - qf))
+            v = c;
+    }
+    if (again)
+    {
+        // the band to the ring, with the marks the ring form keeps
+        __syncwarp();
+        const int s0 = FWD ? -hgh : low;
+        const int p = (lane - s0) & 31;
+        if (low <= hgh && p <= hgh - low)
+        {
+            const int k = FWD ? hgh - p : low + p;
+            const int y = (v - k) >> 1, x = v - y;
+            R.V[0][k & RM] = v;
+            R.T[0][k & RM] = ((unsigned long long)t1 << 32) | t0;
+            R.HA[0][k & RM] = ha;
+            R.HB[0][k & RM] = hb;
+            R.NA[0][k & RM] = FWD ? (divTS(x) + 1) * TS : (divTS(x + TS - 1) - 1) * TS;
+            R.NB[0][k & RM] =
+                FWD ? divTS(y + TS - boff) * TS + boff : (divTS(y + TS - boff - 1) - 1) * TS + boff;
+        }
+        if (lane == 0)
+            w.sm->besty = (besta - kbest) >> 1;
+        __syncwarp();
+    }
+    w.cells += cells;
+    wvars.hgh = hgh;
+    wvars.low = low;
+    wvars.dif = dif;
+    wvars.besta = besta;
+    wvars.lasta = lasta;
+    wvars.npeb = npeb;
+    return again;
 }
 
 // One wave of both teams of a duo warp at once: wave_step's work, for each team on its own
@@ -1560,6 +1880,45 @@ __device__ __forceinline__ void wave_end(const bool FWD, WarpCtx<RG>& w, WaveVar
         *mind = w.sm->span_lo;
 }
 
+// Ring waves out of line, one copy for both directions: the wide waves and the unusual ones, until
+// the band is narrower than back (0: to the end).  The state travels in sm->wv, so that the
+// caller's loop keeps its registers.  Returns whether the wave loop goes on.
+template <int RG>
+__device__ __noinline__ bool wave_ring(const bool fwd, WarpSmem<RG>* sm, int4* peb, int pcap, DevStatus* st, int item,
+                                       int tspace, int ave_path, const int16_t* table, const int16_t* score,
+                                       const uint32_t* apk, uint32_t ag, const uint32_t* bpk, uint32_t bg, int alen,
+                                       int blen, int comp, int minp, int maxp, int back)
+{
+    WarpCtx<RG> w;
+    w.sm = sm;
+    w.peb = peb;
+    w.pcap = pcap;
+    w.st = st;
+    w.lane = lane_id();
+    w.err = 0;
+    w.item = item;
+    w.cells = 0;
+    AlignParams P;
+    P.tspace = tspace;
+    P.ave_path = ave_path;
+    P.table = table;
+    P.score = score;
+    WaveVars v = sm->wv;
+    bool on;
+    do
+        on = wave_step<RG, true>(fwd, w, v, P, nullptr, nullptr, apk, ag, bpk, bg, alen, blen, comp, minp, maxp);
+    while (on && v.hgh - v.low >= back);  // an empty band is wave_step's to report
+    __syncwarp();
+    if (w.lane == 0)
+    {
+        sm->wv = v;
+        sm->wv_err = w.err;
+        sm->wv_cells = w.cells;
+    }
+    __syncwarp();
+    return on;
+}
+
 template <bool FWD, int RG, bool PK>
 __device__ void wave(WarpCtx<RG>& w, const AlignParams& P, const uint8_t* aseq0, const uint8_t* bseq0,
                      const uint32_t* apk, uint32_t ag, const uint32_t* bpk, uint32_t bg, int alen, int blen,
@@ -1570,8 +1929,31 @@ __device__ void wave(WarpCtx<RG>& w, const AlignParams& P, const uint8_t* aseq0,
     wave_begin<RG, PK>(FWD, w, v, P, aseq0, bseq0, apk, ag, bpk, bg, alen, blen, comp, *mind, maxd, mida);
     if (w.err)
         return;
-    while (wave_step<RG, PK>(FWD, w, v, P, aseq0, bseq0, apk, ag, bpk, bg, alen, blen, comp, minp, maxp))
-        ;
+    if constexpr (PK)
+    {
+        // in registers while the band is narrow; in the ring from a wide wave on until it is narrow
+        // again, and for a read against itself (its band stops at the main diagonal).  The
+        // packed reduction of wave_regs holds anti-diagonals below 2^26
+        const bool regs = P.tsmagic && minp == -INT_MAX && maxp == INT_MAX && alen + blen < (1 << 26);
+        const int boff = comp ? blen % P.tspace : 0;
+        while (!regs || wave_regs<FWD, RG>(w, v, P, apk, ag, bpk, bg, alen, blen, boff))
+        {
+            if (w.lane == 0)
+                w.sm->wv = v;
+            __syncwarp();
+            const bool on = wave_ring<RG>(FWD, w.sm, w.peb, w.pcap, w.st, w.item, P.tspace, P.ave_path, P.table,
+                                          P.score, apk, ag, bpk, bg, alen, blen, comp, minp, maxp,
+                                          regs ? REGS_BACK : 0);
+            v = w.sm->wv;
+            w.err = w.sm->wv_err;
+            w.cells += w.sm->wv_cells;
+            if (!on)
+                break;
+        }
+    }
+    else
+        while (wave_step<RG, PK>(FWD, w, v, P, aseq0, bseq0, apk, ag, bpk, bg, alen, blen, comp, minp, maxp))
+            ;
     if (w.err)
         return;
     wave_end<RG, PK>(FWD, w, v, P, aseq0, bseq0, apk, ag, bpk, bg, alen, blen, comp, apath, bpath, mind, mida, atrace,
@@ -2656,7 +3038,9 @@ constexpr int warps_of()
 // record of a read against itself, its Handle_Redundancies; a separate instance, so that
 // daligner's keeps its code layout.
 #ifndef GD_ALIGN_MINB
-#define GD_ALIGN_MINB 6  // CTAs per SM the warp instance is compiled for (80 registers; 7, at 72, spills and runs 9 % slower)
+// CTAs per SM the warp instance is compiled for, with the waves in registers: 7 (72 registers) runs the
+// 121 Mbp block's aligner in 183 ms per orientation, 6 (80) in 199, 8 (64) in 186
+#define GD_ALIGN_MINB 7
 #endif
 
 template <int RG, bool D2 = false>

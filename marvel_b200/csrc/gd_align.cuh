@@ -49,10 +49,18 @@ struct AlignParams
     HitBits hb;
     const int16_t* table;  // TABLE and SCORE trim tables (set_table, dalign/align.c:196-210)
     const int16_t* score;
+    uint32_t tsmagic;      // n / tspace = umulhi(n, tsmagic) for every position n (align_magic); 0: not usable
     int mscore, dscore;    // match / edit weights the tables are built from (align.c:238-240)
     int test_narrow;       // tests only: the main pass runs the TEST_RING instance
     int d2, hgap;          // daligner2's report (dalign2/filter_reporter_cpu.c) and its -H
 };
+
+// tsmagic for reads of up to maxlen bases: with M = floor(2^32 / t) + 1, umulhi(n, M) = n / t while
+// n (M t - 2^32) < 2^32, and M t - 2^32 <= t
+inline uint32_t align_magic(int64_t maxlen, int tspace)
+{
+    return (tspace >= 2 && (maxlen + 2ll * tspace) * tspace < (1ll << 32)) ? (uint32_t)((1ull << 32) / tspace) + 1 : 0;
+}
 
 // Per-warp global scratch, carved from one allocation.
 struct AlignScratch

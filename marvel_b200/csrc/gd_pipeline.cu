@@ -1069,6 +1069,7 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
         return -1;
     const int nwarps_w = c->agrid_w * align_warps_per_cta(1);
     int maxlen = std::max(A.blk.maxlen, B.blk.maxlen);
+    ap.tsmagic = align_magic(maxlen, c->tspace);
     int ptscap = 4 * (2 * (maxlen / c->tspace + 2)) + 32;
     int nbands = ap.maxdiag - ap.mindiag + 8;
     // the instance of each length class (0 warp, 1 wide, 2 duo); daligner2's report has no duo
@@ -2446,6 +2447,7 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     ap.score = P<int16_t>(c->tables) + TRIM_TABLE;
     ap.mscore = c->mscore;
     ap.dscore = c->dscore;
+    ap.tsmagic = align_magic(maxlen, c->tspace);
     int grid = 0;
     if (align_grid(&grid))
         return -1;
