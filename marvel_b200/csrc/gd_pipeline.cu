@@ -13,6 +13,8 @@
 #include <cstring>
 #include <functional>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/gpudalign.h"
@@ -136,6 +138,122 @@ int ensure_host(HostBuf& b, size_t bytes)
     return 0;
 }
 
+// Copies between device memory and pageable host memory through pinned staging: the driver's own
+// pageable path moves one small piece at a time (105 MB of bases took about 25 ms, and results
+// into fresh pages as long again).  STAGE_THREADS host threads take STAGE_CHUNK pieces in turn, each
+// with two pinned buffers, so that one piece's host copy (and the page faults of a fresh result
+// array) runs beside another's transfer.  Small copies and pinned memory go straight.
+constexpr size_t STAGE_CHUNK = 2u << 20;
+constexpr size_t STAGE_MIN = 4u << 20;  // below this the threads cost what they save
+constexpr int STAGE_THREADS = 4;
+
+struct Staging
+{
+    char* buf = nullptr;  // 2 pieces per thread, pinned
+    cudaEvent_t ev[2 * STAGE_THREADS] = {};
+};
+
+void release(Staging& g)
+{
+    for (cudaEvent_t e : g.ev)
+        if (e)
+            cudaEventDestroy(e);
+    if (g.buf)
+        cudaFreeHost(g.buf);
+    g = Staging{};
+}
+
+bool is_pageable(const void* p)
+{
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// dev <-> host (to_dev), n bytes on stream s.  To the device: the host memory may be reused on
+// return, as after a pageable cudaMemcpyAsync.  To the host: complete on return.
+int staged_copy(Staging& g, void* dev, void* host, size_t n, bool to_dev, cudaStream_t s)
+{
+    if (n < STAGE_MIN || !is_pageable(host))
+    {
+        GD_CUDA(cudaMemcpyAsync(to_dev ? dev : host, to_dev ? host : dev, n,
+                                to_dev ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, s));
+        if (!to_dev)
+            GD_CUDA(cudaStreamSynchronize(s));
+        return 0;
+    }
+    if (!g.buf)
+    {
+        for (cudaEvent_t& e : g.ev)
+            GD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        GD_CUDA(cudaMallocHost((void**)&g.buf, 2 * STAGE_THREADS * STAGE_CHUNK));
+    }
+    int dev_id = 0;
+    GD_CUDA(cudaGetDevice(&dev_id));
+    cudaError_t errs[STAGE_THREADS] = {};
+    auto work = [&](int t) {
+        cudaError_t& e = errs[t];
+        if ((e = cudaSetDevice(dev_id)) != cudaSuccess)
+            return;
+        struct
+        {
+            size_t at = 0, len = 0;  // the piece in flight in this buffer
+        } fly[2];
+        auto land = [&](int b) {
+            if (fly[b].len == 0 || e != cudaSuccess)
+                return;
+            e = cudaEventSynchronize(g.ev[2 * t + b]);
+            if (e == cudaSuccess && !to_dev)
+                memcpy((char*)host + fly[b].at, g.buf + (2 * t + b) * STAGE_CHUNK, fly[b].len);
+            fly[b].len = 0;
+        };
+        int b = 0;
+        for (size_t at = t * STAGE_CHUNK; at < n && e == cudaSuccess; at += STAGE_THREADS * STAGE_CHUNK, b ^= 1)
+        {
+            land(b);
+            if (e != cudaSuccess)
+                return;
+            char* const pin = g.buf + (2 * t + b) * STAGE_CHUNK;
+            const size_t len = std::min(STAGE_CHUNK, n - at);
+            if (to_dev)
+            {
+                memcpy(pin, (const char*)host + at, len);
+                e = cudaMemcpyAsync((char*)dev + at, pin, len, cudaMemcpyHostToDevice, s);
+            }
+            else
+                e = cudaMemcpyAsync(pin, (const char*)dev + at, len, cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess)
+                e = cudaEventRecord(g.ev[2 * t + b], s);
+            fly[b].at = at;
+            fly[b].len = len;
+        }
+        land(b);
+        land(b ^ 1);
+    };
+    std::vector<std::thread> th;
+    for (int t = 1; t < STAGE_THREADS; t++)
+    {
+        try
+        {
+            th.emplace_back(work, t);
+        }
+        catch (const std::system_error&)
+        {
+            work(t);  // no thread to be had: its share here
+        }
+    }
+    work(0);
+    for (std::thread& x : th)
+        x.join();
+    for (cudaError_t e : errs)
+        GD_CUDA(e);
+    return 0;
+}
+
 struct Slot
 {
     DevBuf bases, boff, rlen, manno, mdata, pk;
@@ -202,6 +320,7 @@ struct gd_context
     DevBuf acc_rec, acc_tr, srt_rec, srt_tr, okey0, okey1, oval0, oval1, olen;
     uint64_t acc_n = 0, acc_tb = 0, srt_n = 0, srt_tb = 0;
     bool srt_valid = false;
+    Staging stage;        // pageable host memory <-> device
     HostBuf h_rec, h_tr;  // pinned staging for file writes
     DevBuf las_raw, las_off, las_rec, las_out;  // gd_las_sort
     DevBuf lb_a, lb_b, lb_pka, lb_pkb, lb_in, lb_out, lb_tr;  // gd_local_alignment_batch
@@ -1448,6 +1567,7 @@ void gd_destroy(gd_context* c)
     for (HostBuf* h : {&c->h_rec, &c->h_tr})
         if (h->p)
             cudaFreeHost(h->p);
+    release(c->stage);
     for (Slot& s : c->slot)
     {
         DevBuf* sb[] = {&s.bases, &s.boff, &s.rlen, &s.manno, &s.mdata, &s.code, &s.read, &s.rpos};
@@ -1561,7 +1681,8 @@ int gd_load_block(gd_context* c, int slot, const gd_block* b)
     if (ensure(s.bases, nb + 1 + 64) || ensure(s.boff, (b->nreads + 1) * 8) || ensure(s.rlen, b->nreads * 4 + 4))
         return -1;
     GD_CUDA(cudaMemsetAsync(s.bases.p, 4, nb + 1 + 64, c->s));
-    GD_CUDA(cudaMemcpyAsync((uint8_t*)s.bases.p + 32, b->bases - 1, nb + 1, cudaMemcpyHostToDevice, c->s));
+    if (staged_copy(c->stage, (uint8_t*)s.bases.p + 32, (void*)(b->bases - 1), nb + 1, true, c->s))
+        return -1;
     GD_CUDA(cudaMemcpyAsync(s.boff.p, b->boff, (b->nreads + 1) * 8, cudaMemcpyHostToDevice, c->s));
     GD_CUDA(cudaMemcpyAsync(s.rlen.p, b->rlen, b->nreads * 4, cudaMemcpyHostToDevice, c->s));
     s.has_mask = b->mask_anno != nullptr;
@@ -2143,10 +2264,9 @@ int64_t gd_get_overlaps(gd_context* c, gd_overlap* recs, uint8_t* trace, int64_t
     {
         // everything fits: the records and the trace bytes (laid out in record order) in two
         // back-to-back copies
-        GD_CUDA(cudaMemcpyAsync(recs, c->srt_rec.p, (size_t)m * sizeof(gd_overlap), cudaMemcpyDeviceToHost, c->s));
-        if (c->srt_tb)
-            GD_CUDA(cudaMemcpyAsync(trace, c->srt_tr.p, c->srt_tb, cudaMemcpyDeviceToHost, c->s));
-        GD_CUDA(cudaStreamSynchronize(c->s));
+        if (staged_copy(c->stage, c->srt_rec.p, recs, (size_t)m * sizeof(gd_overlap), false, c->s) ||
+            (c->srt_tb && staged_copy(c->stage, c->srt_tr.p, trace, c->srt_tb, false, c->s)))
+            return -1;
         return m;
     }
     // the leading records whose traces fit in tcap
@@ -2312,7 +2432,10 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
     GD_CUDA(cudaMemcpyAsync(c->vf_rec.p, recs, (size_t)n * sizeof(OutRec), cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(c->vf_first.p, first.data(), (size_t)(n + 1) * 8, cudaMemcpyHostToDevice, s));
     if (thi > tlo)
-        GD_CUDA(cudaMemcpyAsync(c->vf_trace.p, trace + tlo, (size_t)(thi - tlo), cudaMemcpyHostToDevice, s));
+    {
+        if (staged_copy(c->stage, c->vf_trace.p, (void*)(trace + tlo), (size_t)(thi - tlo), true, s))
+            return -1;
+    }
     GD_CUDA(cudaMemsetAsync(c->vf_diff.p, 0, (size_t)n * 4, s));
     GD_CUDA(cudaMemsetAsync(c->vf_misc.p, 0, 64, s));
     if (launch_trace_segments(P<OutRec>(c->vf_rec), n, P<int64_t>(c->vf_first), P<uint8_t>(c->vf_trace), tlo, TS, tbytes,
@@ -2473,8 +2596,9 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     // sequences: caller buffers hold [4, read, 4, read, ...] with offsets relative to index 0
     GD_CUDA(cudaMemsetAsync(c->lb_a.p, 4, alen_total + 128, s));
     GD_CUDA(cudaMemsetAsync(c->lb_b.p, 4, blen_total + 128, s));
-    GD_CUDA(cudaMemcpyAsync(P<uint8_t>(c->lb_a) + 64, abases, alen_total, cudaMemcpyHostToDevice, s));
-    GD_CUDA(cudaMemcpyAsync(P<uint8_t>(c->lb_b) + 64, bbases, blen_total, cudaMemcpyHostToDevice, s));
+    if (staged_copy(c->stage, P<uint8_t>(c->lb_a) + 64, (void*)abases, alen_total, true, s) ||
+        staged_copy(c->stage, P<uint8_t>(c->lb_b) + 64, (void*)bbases, blen_total, true, s))
+        return -1;
     GD_CUDA(cudaMemcpyAsync(d_ao, aoff, n8, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_bo, boff, n8, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_al, alen, n4, cudaMemcpyHostToDevice, s));
@@ -2497,7 +2621,8 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
         return -1;
     }
     GD_CUDA(cudaMemcpyAsync(out12, d_out, 12 * n4, cudaMemcpyDeviceToHost, s));
-    GD_CUDA(cudaMemcpyAsync(trace, c->lb_tr.p, (size_t)nseeds * trstride * 2, cudaMemcpyDeviceToHost, s));
+    if (staged_copy(c->stage, c->lb_tr.p, trace, (size_t)nseeds * trstride * 2, false, s))
+        return -1;
     GD_CUDA(cudaMemcpyAsync(cells, d_cells, n8, cudaMemcpyDeviceToHost, s));
     GD_CUDA(cudaStreamSynchronize(s));
     return 0;
@@ -2573,11 +2698,10 @@ int gd_mlp_forward(gd_context* c, const float* params, const float* feat, int64_
         return -1;
     cudaStream_t s = c->s;
     GD_CUDA(cudaMemcpyAsync(c->tri_w.p, params, gd::TRI_NPARAM * 4, cudaMemcpyHostToDevice, s));
-    GD_CUDA(cudaMemcpyAsync(c->tri_x.p, feat, (size_t)n * gd::TRI_NF * 4, cudaMemcpyHostToDevice, s));
-    if (gd::launch_mlp_forward(P<float>(c->tri_w), P<float>(c->tri_x), n, P<float>(c->tri_prob), s))
+    if (staged_copy(c->stage, c->tri_x.p, (void*)feat, (size_t)n * gd::TRI_NF * 4, true, s) ||
+        gd::launch_mlp_forward(P<float>(c->tri_w), P<float>(c->tri_x), n, P<float>(c->tri_prob), s) ||
+        staged_copy(c->stage, c->tri_prob.p, prob, (size_t)n * 4, false, s))
         return -1;
-    GD_CUDA(cudaMemcpyAsync(prob, c->tri_prob.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
-    GD_CUDA(cudaStreamSynchronize(s));
     return 0;
 }
 
