@@ -2948,6 +2948,84 @@ __device__ __forceinline__ int first_above(const uint64_t* hkey, int lo, int hi,
     return lo;
 }
 
+// The panel band scores (filter.c:1754-1766) of hits [lidx, nend), lane-parallel: the hits of a
+// chunk of 32 are grouped by diagonal band, each hit's predecessor in its band comes by shuffle
+// (from lastp for a group's first), and one lane adds the group's sum.
+__device__ __forceinline__ void panel_scores(const uint64_t* __restrict__ hkey, const uint32_t* __restrict__ hdiag,
+                                             int lidx, int nend, int lane, unsigned lt, int K, int BS,
+                                             const HitBits& hb, int* score, int* lastp)
+{
+    for (int base = lidx; base < nend; base += 32)
+    {
+        int i = base + lane;
+        bool valid = i < nend;
+        int ap = 0, dg = 0;
+        if (valid)
+        {
+            ap = hit_apos(hkey[i], hb);
+            dg = ((int)hdiag[i]) >> BS;
+        }
+        unsigned key = valid ? (unsigned)dg : (0x80000000u | (unsigned)lane);
+        unsigned peers = __match_any_sync(GD_FULL, key);
+        unsigned lower = peers & lt;
+        int src = lower ? 31 - __clz(lower) : lane;
+        int prevap = __shfl_sync(GD_FULL, ap, src);
+        int delta = 0;
+        if (valid)
+        {
+            int prev = lower ? prevap : lastp[dg];
+            delta = (ap - prev >= K) ? K : ap - prev;
+        }
+        unsigned todo = __ballot_sync(GD_FULL, valid);
+        while (todo)
+        {
+            int leader = __ffs(todo) - 1;
+            unsigned grpm = __shfl_sync(GD_FULL, peers, leader);
+            int sum = __reduce_add_sync(GD_FULL, ((grpm >> lane) & 1) ? delta : 0);
+            int last = 31 - __clz(grpm);
+            int lastap = __shfl_sync(GD_FULL, ap, last);
+            int gdg = __shfl_sync(GD_FULL, dg, leader);
+            if (lane == 0)
+            {
+                score[gdg] += sum;
+                lastp[gdg] = lastap;
+            }
+            todo &= ~grpm;
+        }
+        __syncwarp();
+    }
+}
+
+// A seed aligned ahead of this kernel, as local_alignment leaves it: both paths in shared memory,
+// their traces in the warp's points, the cells in sm->wv_cells.  False when there is none.
+template <int RG>
+__device__ __noinline__ bool take_ahead(WarpSmem<RG>* sm, uint16_t* pts, int ptscap, int lane,
+                                        const AheadPath* __restrict__ path, int n, const uint16_t* __restrict__ trace,
+                                        int diag, int apos)
+{
+    for (int base = 0; base < n; base += 32)
+    {
+        const int i = base + lane;
+        const unsigned m = __ballot_sync(GD_FULL, i < n && path[i].diag == diag && path[i].apos == apos);
+        if (!m)
+            continue;
+        const AheadPath p = path[base + __ffs(m) - 1];
+        if (!p.ok || p.atlen + p.btlen > ptscap)
+            return false;
+        if (lane == 0)
+        {
+            sm->ap = LAPath{p.abpos, p.bbpos, p.aepos, p.bepos, p.diffs, p.atlen, 0, 0};
+            sm->bp = LAPath{p.b_abpos, p.b_bbpos, p.b_aepos, p.b_bepos, p.diffs, p.btlen, p.atlen, 0};
+            sm->wv_cells = p.cells;
+        }
+        for (int k = lane; k < p.atlen + p.btlen; k += 32)
+            pts[k] = trace[p.at + k];
+        __syncwarp();
+        return true;
+    }
+    return false;
+}
+
 template <int RG>
 __device__ void store_path(WarpCtx<RG>& w, const LAPath& lp, MPath* dst, PairBuf& pb)
 {
@@ -3036,14 +3114,16 @@ constexpr int warps_of()
 
 // D2: daligner2's report (dalign2/filter_reporter_cpu.c) -- its -H, its rule for the B-side
 // record of a read against itself, its Handle_Redundancies; a separate instance, so that
-// daligner's keeps its code layout.
+// daligner's keeps its code layout.  AHEAD: some groups have seeds aligned ahead (an instance of its
+// own for the same reason: with the look-up in the plain one the 121 Mbp block took 188 ms
+// instead of 183).
 #ifndef GD_ALIGN_MINB
 // CTAs per SM the warp instance is compiled for, with the waves in registers: 7 (72 registers) runs the
 // 121 Mbp block's aligner in 183 ms per orientation, 6 (80) in 199, 8 (64) in 186
 #define GD_ALIGN_MINB 7
 #endif
 
-template <int RG, bool D2 = false>
+template <int RG, bool D2 = false, bool AHEAD = false>
 __global__ void __launch_bounds__(warps_of<RG>() * 32, RG == WIDE_RING ? 1 : GD_ALIGN_MINB)
     k_align_pairs(DevBlock A, DevBlock B, const uint64_t* __restrict__ hkey, const uint32_t* __restrict__ hdiag,
                   const uint2* __restrict__ groups, const uint32_t* __restrict__ order, unsigned ngroups, AlignParams P,
@@ -3114,6 +3194,8 @@ __global__ void __launch_bounds__(warps_of<RG>() * 32, RG == WIDE_RING ? 1 : GD_
         pb.err = 0;
         int novla = 0, novlb = 0;
         int tlo = INT_MAX, thi = INT_MIN;  // lasta bands touched in this pair
+        // its seeds aligned ahead
+        const uint2 ahead = AHEAD && g < (unsigned)AHEAD_GROUPS ? out.ahead.groups[g] : make_uint2(0, 0);
 
         int nidx = s, amark2 = 0;
         while (nidx < e && !w.err && !pb.err)
@@ -3129,46 +3211,7 @@ __global__ void __launch_bounds__(warps_of<RG>() * 32, RG == WIDE_RING ? 1 : GD_
                 nidx = h2;
                 continue;
             }
-            // panel band scores (filter.c:1754-1766)
-            for (int base = lidx; base < nend; base += 32)
-            {
-                int i = base + lane;
-                bool valid = i < nend;
-                int ap = 0, dg = 0;
-                if (valid)
-                {
-                    ap = hit_apos(hkey[i], P.hb);
-                    dg = ((int)hdiag[i]) >> BS;
-                }
-                unsigned key = valid ? (unsigned)dg : (0x80000000u | (unsigned)lane);
-                unsigned peers = __match_any_sync(GD_FULL, key);
-                unsigned lower = peers & lt;
-                int src = lower ? 31 - __clz(lower) : lane;
-                int prevap = __shfl_sync(GD_FULL, ap, src);
-                int delta = 0;
-                if (valid)
-                {
-                    int prev = lower ? prevap : lastp[dg];
-                    delta = (ap - prev >= K) ? K : ap - prev;
-                }
-                unsigned todo = __ballot_sync(GD_FULL, valid);
-                while (todo)
-                {
-                    int leader = __ffs(todo) - 1;
-                    unsigned grpm = __shfl_sync(GD_FULL, peers, leader);
-                    int sum = __reduce_add_sync(GD_FULL, ((grpm >> lane) & 1) ? delta : 0);
-                    int last = 31 - __clz(grpm);
-                    int lastap = __shfl_sync(GD_FULL, ap, last);
-                    int gdg = __shfl_sync(GD_FULL, dg, leader);
-                    if (lane == 0)
-                    {
-                        score[gdg] += sum;
-                        lastp[gdg] = lastap;
-                    }
-                    todo &= ~grpm;
-                }
-                __syncwarp();
-            }
+            panel_scores(hkey, hdiag, lidx, nend, lane, lt, K, BS, P.hb, score, lastp);
             // seeds in hit order (filter.c:1776-1893)
             for (int base = lidx; base < nend && !w.err && !pb.err; base += 32)
             {
@@ -3196,8 +3239,12 @@ __global__ void __launch_bounds__(warps_of<RG>() * 32, RG == WIDE_RING ? 1 : GD_
                         continue;
                     nseeds++;
                     int bpj = apj - dj;
-                    local_alignment<RG, true>(w, P, aseq, bseq, A.pk, ag, B.pk, bg, alen, blen, P.comp, dj,
-                                              apj + bpj);
+                    if (AHEAD && ahead.y && take_ahead<RG>(w.sm, w.pts, w.ptscap, lane, out.ahead.path + ahead.x,
+                                                           (int)ahead.y, out.ahead.trace, dj, apj))
+                        w.cells += w.sm->wv_cells;
+                    else
+                        local_alignment<RG, true>(w, P, aseq, bseq, A.pk, ag, B.pk, bg, alen, blen, P.comp, dj,
+                                                  apj + bpj);
                     if (w.err)
                         break;
                     const LAPath apth = w.sm->ap;
@@ -3921,6 +3968,10 @@ void align_scratch_carve(AlignScratch* s, void* base, int nwarps, int pcap, int 
     s->btr = btcap ? (uint16_t*)p : nullptr;
 }
 
+__global__ void k_ahead_align(DevBlock A, DevBlock B, const uint64_t* __restrict__ hkey,
+                              const uint2* __restrict__ groups, AlignParams P, AlignScratch sc, Ahead ah,
+                              DevStatus* st);
+
 // Prefer the smallest shared-memory carveout that holds ctas CTAs of kern: the rest of the SM's
 // 256 KB stays L1, which the aligner's reads of the 2-bit words, the pebbles and the trim tables
 // depend on
@@ -3945,7 +3996,9 @@ int align_grid(int* grid_out, int wide)
     {
         if (prefer_l1((const void*)k_align_pairs<RING>, GD_ALIGN_MINB) ||
             prefer_l1((const void*)k_align_pairs<RING, true>, GD_ALIGN_MINB) ||
-            prefer_l1((const void*)k_align_pairs<TEST_RING>, GD_ALIGN_MINB))
+            prefer_l1((const void*)k_align_pairs<TEST_RING>, GD_ALIGN_MINB) ||
+            prefer_l1((const void*)k_align_pairs<RING, false, true>, GD_ALIGN_MINB) ||
+            prefer_l1((const void*)k_ahead_align, GD_ALIGN_MINB))
             return -1;
         carved = true;
     }
@@ -3999,9 +4052,206 @@ int launch_align_pairs(const DevBlock& A, const DevBlock& B, const uint64_t* hke
     else if (p.test_narrow)
         k_align_pairs<TEST_RING><<<grid, ALIGN_WARPS * 32, 0, s>>>(A, B, hkey, hdiag, groups, order, ngroups, p, sc,
                                                                    out, queue, st);
+    else if (out.ahead.groups)
+        k_align_pairs<RING, false, true><<<grid, ALIGN_WARPS * 32, 0, s>>>(A, B, hkey, hdiag, groups, order, ngroups, p,
+                                                                          sc, out, queue, st);
     else
         k_align_pairs<RING><<<grid, ALIGN_WARPS * 32, 0, s>>>(A, B, hkey, hdiag, groups, order, ngroups, p, sc, out,
                                                               queue, st);
+    GD_LAUNCHED(1);
+    GD_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// ------------------------------------------------------------------------------------------
+// Seeds aligned ahead.  A pair group's seeds are aligned one after the other, because each
+// alignment moves lasta, which decides the next.  In a group of two reads that share a tandem
+// repeat (thousands of hits, a hundred alignments) that chain outlasts everything else in the
+// block: a 53 Mbp block pair kept one warp busy for 100 ms where its whole work is worth 40 (aligned
+// ahead: 90 and 107 ms of aligner per orientation become 70 and 78).  But
+// lasta is 0 on a band no alignment has touched, so the first candidate of every band is a
+// likely seed: these are aligned here first, each on a warp of its own, and the pair kernel,
+// running the same scan as ever, takes a seed's result if it is there (four in five are).  Seeds
+// that turn out to be covered are work for nothing, so only groups with a large share of the
+// block's hits (the host's rule) and a candidate on many bands are treated so.
+// ------------------------------------------------------------------------------------------
+
+// The seeds: a warp per place of the order.
+__global__ void __launch_bounds__(ALIGN_WARPS * 32)
+    k_ahead_seeds(const uint64_t* __restrict__ hkey, const uint32_t* __restrict__ hdiag,
+                  const uint2* __restrict__ groups, const uint32_t* __restrict__ order, unsigned nheavy,
+                  const uint8_t* __restrict__ skip, AlignParams P, AlignScratch sc, Ahead ah)
+{
+    __shared__ int2 found[ALIGN_WARPS][AHEAD_SEEDS];
+    int2* const mine = found[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const unsigned g = blockIdx.x * ALIGN_WARPS + (threadIdx.x >> 5);
+    if (g >= nheavy || g >= (unsigned)sc.nwarps)
+        return;
+    const unsigned item = order[g];
+    if (skip && skip[item])
+        return;
+    const uint2 grp = groups[item];
+    int* score = sc.bands + (size_t)g * 3 * sc.nbands - (P.mindiag - 2);
+    int* lastp = score + sc.nbands;
+    int* seen = lastp + sc.nbands;  // bands that have a seed
+    const int K = P.kmer, BS = P.binshift;
+    const int minhit = (P.hitmin - 1) / K + 1;
+    const unsigned lt = lanemask_lt();
+    const int s = (int)grp.x, e = (int)grp.y;
+    unsigned n = 0;
+    int nidx = s, amark2 = 0;
+    while (nidx < e)
+    {
+        const int amark = amark2 + PANEL_SIZE;
+        amark2 = amark - PANEL_OVERLAP;
+        const int lidx = nidx;
+        const int q = first_above(hkey, lidx, e, amark, P.hb);
+        const int nend = (q < e) ? q + 1 : e;
+        const int h2 = first_above(hkey, lidx, nend, amark2, P.hb);
+        if (nend - lidx >= minhit)
+        {
+            panel_scores(hkey, hdiag, lidx, nend, lane, lt, K, BS, P.hb, score, lastp);
+            for (int base = lidx; base < nend; base += 32)
+            {
+                const int i = base + lane;
+                int ap = 0, d = 0, dg = 0;
+                bool fresh = false;
+                if (i < nend)
+                {
+                    ap = hit_apos(hkey[i], P.hb);
+                    d = (int)hdiag[i];
+                    dg = d >> BS;
+                    const int sc0 = score[dg];
+                    fresh = ((sc0 + score[dg + 1] >= P.hitmin) || (sc0 + score[dg - 1] >= P.hitmin)) && ap > 0 &&
+                            seen[dg] == 0;
+                }
+                // the first of each band
+                const unsigned peers = __match_any_sync(GD_FULL, fresh ? (unsigned)dg : (0x80000000u | (unsigned)lane));
+                fresh = fresh && !(peers & lt);
+                const unsigned m = __ballot_sync(GD_FULL, fresh);
+                if (fresh)
+                {
+                    seen[dg] = 1;
+                    const unsigned t = n + __popc(m & lt);
+                    if (t < (unsigned)AHEAD_SEEDS)
+                        mine[t] = make_int2(d, ap);
+                }
+                n += __popc(m);
+                __syncwarp();
+            }
+            for (int i = lidx + lane; i < nend; i += 32)
+            {
+                const int dg = ((int)hdiag[i]) >> BS;
+                score[dg] = 0;
+                lastp[dg] = 0;
+            }
+            __syncwarp();
+        }
+        nidx = h2;
+    }
+    for (int i = s + lane; i < e; i += 32)
+        seen[((int)hdiag[i]) >> BS] = 0;
+    n = min(n, (unsigned)AHEAD_SEEDS);
+    if (n < (unsigned)AHEAD_BANDS)
+        return;
+    unsigned first = 0;
+    if (lane == 0)
+        first = atomicAdd(&ah.ctr[0], n);
+    first = __shfl_sync(GD_FULL, first, 0);
+    const bool room = first + n <= (unsigned)AHEAD_CAP;
+    for (unsigned t = lane; t < n && first + t < (unsigned)AHEAD_CAP; t += 32)
+    {
+        AheadPath& p = ah.path[first + t];
+        p.item = room ? (int)item : -1;
+        p.diag = mine[t].x;
+        p.apos = mine[t].y;
+        p.ok = 0;
+    }
+    if (lane == 0 && room)
+        ah.groups[g] = make_uint2(first, n);
+}
+
+// Their alignments: persistent warps
+__global__ void __launch_bounds__(ALIGN_WARPS * 32, GD_ALIGN_MINB)
+    k_ahead_align(DevBlock A, DevBlock B, const uint64_t* __restrict__ hkey, const uint2* __restrict__ groups,
+                  AlignParams P, AlignScratch sc, Ahead ah, DevStatus* st)
+{
+    __shared__ WarpSmem<RING> smem[ALIGN_WARPS];
+    const int lane = threadIdx.x & 31;
+    const int wib = threadIdx.x >> 5;
+    const int gw = blockIdx.x * ALIGN_WARPS + wib;
+    if (gw >= sc.nwarps)
+        return;
+    WarpCtx<RING> w;
+    w.sm = &smem[wib];
+    w.peb = sc.peb + (size_t)gw * sc.pcap;
+    w.pcap = sc.pcap;
+    w.pts = sc.pts + (size_t)gw * sc.ptscap;
+    w.ptscap = sc.ptscap;
+    w.st = st;
+    w.lane = lane;
+    const unsigned total = min(ah.ctr[0], (unsigned)AHEAD_CAP);
+    while (true)
+    {
+        unsigned q = 0;
+        if (lane == 0)
+            q = atomicAdd(&ah.ctr[1], 1u);
+        q = __shfl_sync(GD_FULL, q, 0);
+        if (q >= total)
+            break;
+        AheadPath* const out = ah.path + q;
+        const int item = out->item;
+        if (item < 0)
+            continue;
+        const uint64_t key = hkey[groups[item].x];
+        const int ar = (int)((key >> P.hb.pbits) & ((1ull << P.hb.abits) - 1));
+        const int br = (int)(key >> (P.hb.pbits + P.hb.abits));
+        const int diag = out->diag, apos = out->apos;
+        w.err = 0;
+        w.cells = 0;
+        w.item = item;
+        local_alignment<RING, true>(w, P, A.bases + A.boff[ar], B.bases + B.boff[br], A.pk,
+                                    PK_BIAS + (uint32_t)A.boff[ar], B.pk, PK_BIAS + (uint32_t)B.boff[br], A.rlen[ar],
+                                    B.rlen[br], P.comp, diag, 2 * apos - diag);
+        __syncwarp();
+        if (w.err)
+            continue;
+        const LAPath a = w.sm->ap, b = w.sm->bp;
+        unsigned long long t0 = 0;
+        if (lane == 0)
+            t0 = atomicAdd(ah.top, (unsigned long long)(a.tlen + b.tlen));
+        t0 = __shfl_sync(GD_FULL, t0, 0);
+        if (t0 + a.tlen + b.tlen > ah.cap)
+            continue;
+        for (int i = lane; i < a.tlen; i += 32)
+            ah.trace[t0 + i] = w.pts[a.toff + i];
+        for (int i = lane; i < b.tlen; i += 32)
+            ah.trace[t0 + a.tlen + i] = w.pts[b.toff + i];
+        if (lane == 0)
+            *out = AheadPath{item,    diag,    apos,    1,       a.abpos, a.bbpos, a.aepos, a.bepos, a.diffs,
+                             a.tlen,  b.abpos, b.bbpos, b.aepos, b.bepos, b.tlen,  w.cells, t0};
+        __syncwarp();
+    }
+}
+
+int launch_align_ahead(const DevBlock& A, const DevBlock& B, const uint64_t* hkey, const uint32_t* hdiag,
+                       const uint2* groups, const uint32_t* order, unsigned nheavy, const uint8_t* skip, AlignParams p,
+                       AlignScratch sc, Ahead ah, DevStatus* st, int grid, cudaStream_t s, bool* any)
+{
+    GD_CUDA(cudaMemsetAsync(ah.groups, 0, AHEAD_GROUPS * sizeof(uint2) + 16, s));  // ctr and top follow groups
+    const unsigned n = nheavy < (unsigned)AHEAD_GROUPS ? nheavy : (unsigned)AHEAD_GROUPS;
+    k_ahead_seeds<<<(n + ALIGN_WARPS - 1) / ALIGN_WARPS, ALIGN_WARPS * 32, 0, s>>>(hkey, hdiag, groups, order, n, skip, p,
+                                                                                  sc, ah);
+    GD_LAUNCHED(1);
+    GD_CUDA(cudaGetLastError());
+    unsigned nseeds = 0;
+    GD_CUDA(cudaMemcpyAsync(&nseeds, ah.ctr, 4, cudaMemcpyDeviceToHost, s));
+    GD_CUDA(cudaStreamSynchronize(s));
+    *any = nseeds > 0;
+    if (nseeds == 0)
+        return 0;
+    k_ahead_align<<<grid, ALIGN_WARPS * 32, 0, s>>>(A, B, hkey, groups, p, sc, ah, st);
     GD_LAUNCHED(1);
     GD_CUDA(cudaGetLastError());
     return 0;

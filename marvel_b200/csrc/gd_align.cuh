@@ -82,6 +82,33 @@ struct AlignScratch
     int btcap;
 };
 
+// Seeds of the heaviest pair groups aligned ahead of the pair kernel, one per warp (gd_align.cu,
+// k_ahead_seeds).  Groups are named by their place in the order (the heaviest come first).
+constexpr int AHEAD_GROUPS = 4096;    // places of the order looked at
+constexpr int AHEAD_SEEDS = 256;      // seeds of a group at most,
+constexpr int AHEAD_BANDS = 12;       // and at least: an overlap that is no repeat has fewer bands with a candidate
+constexpr int AHEAD_CAP = 1 << 18;    // seeds of all groups
+constexpr int AHEAD_MIN_HITS = 512;
+
+struct AheadPath
+{
+    int32_t item, diag, apos, ok;  // the pair group (-1: none) and the seed; whether its alignment is here
+    int32_t abpos, bbpos, aepos, bepos, diffs, atlen;    // A path
+    int32_t b_abpos, b_bbpos, b_aepos, b_bepos, btlen;   // B path
+    uint32_t cells;
+    uint64_t at;                   // its traces: A's values, then B's
+};
+
+struct Ahead
+{
+    uint2* groups;      // (first, count) of a group's seeds in path [AHEAD_GROUPS]; null: none are aligned ahead
+    AheadPath* path;    // [AHEAD_CAP]
+    unsigned* ctr;      // [0] seeds, [1] queue; right behind groups, top behind them
+    unsigned long long* top;  // trace values used
+    uint16_t* trace;
+    unsigned long long cap;
+};
+
 struct AlignOut
 {
     OutRec* rec;
@@ -92,6 +119,7 @@ struct AlignOut
     uint2* gstat;         // per pair group: (records emitted, wave cells) (may be null)
     unsigned* wide_list;  // groups handed to the wide instance (null: a too-wide band is an error)
     unsigned* nwide;      // their count
+    Ahead ahead;
 };
 
 size_t align_scratch_bytes(int nwarps, int pcap, int ptscap, int mcap, int tcap, int nbands, int bvcap = 0,
@@ -108,6 +136,14 @@ void align_scratch_carve(AlignScratch* s, void* base, int nwarps, int pcap, int 
 int launch_align_pairs(const DevBlock& A, const DevBlock& B, const uint64_t* hkey, const uint32_t* hdiag,
                        const uint2* groups, const uint32_t* order, unsigned ngroups, AlignParams p, AlignScratch sc,
                        AlignOut out, unsigned* queue, DevStatus* st, int grid, cudaStream_t s, int wide = 0);
+
+// Aligns the likely seeds of the order's first nheavy groups (at most AHEAD_GROUPS) before
+// launch_align_pairs of the same order takes them.  st: a status of its own (a seed that fails
+// here is aligned by the pair kernel).  *any: whether there were seeds (without, the pair kernel runs
+// its plain instance).
+int launch_align_ahead(const DevBlock& A, const DevBlock& B, const uint64_t* hkey, const uint32_t* hdiag,
+                       const uint2* groups, const uint32_t* order, unsigned nheavy, const uint8_t* skip, AlignParams p,
+                       AlignScratch sc, Ahead ah, DevStatus* st, int grid, cudaStream_t s, bool* any);
 
 // One Local_Alignment per seed (for parity tests of the wave alone).  out12 per seed:
 // A-path {abpos,bbpos,aepos,bepos,diffs,tlen}, B-path the same; traces at

@@ -817,10 +817,11 @@ __global__ void __launch_bounds__(FT) k_select_groups(const uint32_t* __restrict
                                                      const uint32_t* __restrict__ hdiag, int binshift, int kmer,
                                                      int hitmin, HitBits hb, const int32_t* __restrict__ arlen,
                                                      const int32_t* __restrict__ brlen, uint2* groups, uint32_t* cost,
-                                                     uint32_t* idx, unsigned int* ngroups, bool byhits)
+                                                     uint32_t* idx, unsigned int* ngroups, bool byhits,
+                                                     unsigned heavy)
 {
     int64_t g = (int64_t)blockIdx.x * FT + threadIdx.x;
-    bool take = false;
+    bool take = false, many = false;
     uint32_t s = 0, e = 0, c = 0;
     if (g < nstarts)
     {
@@ -837,9 +838,15 @@ __global__ void __launch_bounds__(FT) k_select_groups(const uint32_t* __restrict
             // of alen + blen) are a repeat's, aligned many times by its one warp: such a group
             // starts first.  A 53 Mbp block pair with tandem repeats: forward aligner 95 -> 88 ms
             if (byhits)
-                c = max(c, (uint32_t)min(16ull * (e - s), 0x7fffffffull));
+                c = max(c, (uint32_t)min(16ull * (e - s), 0x3fffffffull));
+            // and those whose seeds may be aligned ahead come before all others
+            many = heavy && e - s >= heavy && 32ull * (e - s) > (uint64_t)arlen[ar] + brlen[br];
+            if (many)
+                c = 0x40000000u + min(e - s, 0x3fffffffu);
         }
     }
+    if (many)
+        atomicAdd(ngroups + 1, 1u);
     // slots for the block's kept groups: one atomic per block (a per-warp atomic on the one
     // counter serialised millions of times on the large block pairs)
     __shared__ unsigned wn[FT / 32];
@@ -871,14 +878,14 @@ __global__ void __launch_bounds__(FT) k_select_groups(const uint32_t* __restrict
 int launch_select_groups(const uint32_t* starts, int64_t nstarts, int64_t nhits, int minhit, const uint64_t* hkey,
                          const uint32_t* hdiag, int binshift, int kmer, int hitmin, HitBits hb, const int32_t* arlen,
                          const int32_t* brlen, uint2* groups, uint32_t* cost, uint32_t* idx, unsigned int* ngroups,
-                         bool byhits, cudaStream_t s)
+                         bool byhits, unsigned heavy, cudaStream_t s)
 {
-    GD_CUDA(cudaMemsetAsync(ngroups, 0, sizeof(unsigned), s));
+    GD_CUDA(cudaMemsetAsync(ngroups, 0, 2 * sizeof(unsigned), s));
     if (nstarts <= 0)
         return 0;
     k_select_groups<<<(unsigned)gd_cdiv<int64_t>(nstarts, FT), FT, 0, s>>>(
         starts, nstarts, nhits, minhit, hkey, hdiag, binshift, kmer, hitmin, hb, arlen, brlen, groups, cost, idx, ngroups,
-        byhits);
+        byhits, heavy);
     GD_LAUNCHED(1);
     GD_CUDA(cudaGetLastError());
     return 0;

@@ -140,13 +140,15 @@ int launch_hit_unpack(const uint64_t* packed, int64_t n, HitBits hb, uint64_t* h
 // candidate seed in it (group_can_fire): such a group fires no Local_Alignment and yields
 // nothing, the scan would only have read its hits.  hitmin = 0 keeps every group with >=
 // minhit hits.  The order's cost is alen + blen, with byhits at least 16 times the group's hits (see
-// k_select_groups).
+// k_select_groups); groups of at least heavy hits, and of a hit per 32 bases of
+// alen + blen, come before all others (heavy 0: none do).  ngroups[0] counts the groups kept,
+// ngroups[1] those.
 int launch_pair_flags(const uint64_t* hkey, int64_t n, int pbits, uint32_t* flags, cudaStream_t s);
 int launch_pair_scatter(const uint32_t* flags, const uint32_t* pos, int64_t n, uint32_t* starts, cudaStream_t s);
 int launch_select_groups(const uint32_t* starts, int64_t nstarts, int64_t nhits, int minhit, const uint64_t* hkey,
                          const uint32_t* hdiag, int binshift, int kmer, int hitmin, HitBits hb, const int32_t* arlen,
                          const int32_t* brlen, uint2* groups, uint32_t* cost, uint32_t* idx, unsigned int* ngroups,
-                         bool byhits, cudaStream_t s);
+                         bool byhits, unsigned heavy, cudaStream_t s);
 
 // groups longer than this pass selection untested (the test is quadratic in the hits, and a
 // thread's long group would hold up its warp); nearly all groups without a candidate are shorter

@@ -301,6 +301,7 @@ struct gd_context
     DevBuf ascr_w, wide;  // the wide aligner instance's scratch, and its group list + count
     int agrid_w = 0;
     DevBuf ascr_d;        // the duo instance's scratch
+    DevBuf ah_path, ah_misc, ah_trace;  // seeds aligned ahead of the aligner
     int agrid_d = 0;
     int test_narrow = 0;  // tests only: the main aligner pass with the 32-diagonal instance
     // aligner schedule: empty = every pair group in one persistent launch (longest first from
@@ -1007,6 +1008,9 @@ static int match_filter_d2_t(gd_context* c, int bslot, int cslot, int self)
     return 0;
 }
 
+// trace values of the seeds aligned ahead of one orientation (a seed without room is left to the aligner)
+constexpr size_t AHEAD_TRACE = 48u << 20;
+
 // The hits of one orientation in (hk0, hd0), in generation order, through the hit sort, the
 // pair groups, the learned triage and the seed scan + alignment; records are appended to the
 // overlap buffer in HBM.  c->ev0 marks the start of this orientation's merge stage.
@@ -1091,17 +1095,29 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
     }
     if (launch_pair_scatter(pflags, ppos, nhits, P<uint32_t>(c->starts), s))
         return -1;
+    // groups with at least minhits hits may have their seeds aligned ahead (0: none): a quarter of a
+    // resident warp's share of all hits, from where on a group's chain of alignments can outlast
+    // the rest (on a 53 Mbp block pair groups of 900 hits made 25 alignments, 50 ms), and not in
+    // a small block, whose time is its longest single alignment
+    unsigned minhits = 0;
+    if (!c->agrid && align_grid(&c->agrid, 0))
+        return -1;
+    if (c->variant == 1 && c->sched_edges.empty() && (c->sched_kind.empty() || c->sched_kind[0] == 0) &&
+        !c->test_narrow && nhits >= 128ull * AHEAD_MIN_HITS)
+        minhits = (unsigned)std::max<uint64_t>(AHEAD_MIN_HITS,
+                                               nhits / (4ull * c->agrid * align_warps_per_cta(0)));
     // groups in which daligner's seed scan would find no candidate are dropped here, exactly
     // (daligner2's report keeps its own selection)
     const int minhit = (c->hitmin - 1) / c->kmer + 1;
     const int seed_test = c->variant == 1 ? c->hitmin : 0;
     if (launch_select_groups(P<uint32_t>(c->starts), nst, nhits, minhit, hkey, hdiag, c->binshift, c->kmer, seed_test,
                              hb, P<int32_t>(A.rlen), P<int32_t>(B.rlen), P<uint2>(c->groups), P<uint32_t>(c->gcost),
-                             P<uint32_t>(c->gidx), d_ng, c->sched_edges.empty(), s))
+                             P<uint32_t>(c->gidx), d_ng, c->sched_edges.empty(), minhits, s))
         return -1;
-    unsigned ng = 0;
-    GD_CUDA(cudaMemcpyAsync(&ng, d_ng, 4, cudaMemcpyDeviceToHost, s));
+    unsigned ngh[2] = {0, 0};
+    GD_CUDA(cudaMemcpyAsync(ngh, d_ng, 8, cudaMemcpyDeviceToHost, s));
     GD_CUDA(cudaStreamSynchronize(s));
+    const unsigned ng = ngh[0], nheavy = ngh[1];
     c->stats.groups[oi] = ng;
     if (triage &&
         launch_triage_groups(P<uint2>(c->groups), ng, hkey, hdiag, hb, A.blk, B.blk, comp, c->minover, c->binshift,
@@ -1231,8 +1247,28 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
         unsigned* d_nwide = wide_list + ng;
         GD_CUDA(cudaMemsetAsync(d_nwide, 0, 4, s));
         AlignOut out{P<OutRec>(c->outrec), P<uint8_t>(c->outtr), P<unsigned long long>(c->counters), c->rcap,
-                     c->tbcap, skip, c->tri_collect ? P<uint2>(c->tri_gstat) : nullptr, wide_list, d_nwide};
+                     c->tbcap, skip, c->tri_collect ? P<uint2>(c->tri_gstat) : nullptr, wide_list, d_nwide,
+                     Ahead{}};
         GD_CUDA(cudaEventRecord(c->ev0, s));
+        if (nheavy)
+        {
+            bool any = false;
+            Ahead ah{};
+            ah.cap = AHEAD_TRACE;
+            if (ensure(c->ah_path, AHEAD_CAP * sizeof(AheadPath)) || ensure(c->ah_trace, AHEAD_TRACE * 2) ||
+                ensure(c->ah_misc, AHEAD_GROUPS * sizeof(uint2) + 16 + sizeof(DevStatus)))
+                return -1;
+            ah.path = P<AheadPath>(c->ah_path);
+            ah.trace = P<uint16_t>(c->ah_trace);
+            ah.groups = P<uint2>(c->ah_misc);
+            ah.ctr = (unsigned*)(ah.groups + AHEAD_GROUPS);
+            ah.top = (unsigned long long*)(ah.ctr + 2);
+            if (launch_align_ahead(A.blk, B.blk, hkey, hdiag, P<uint2>(c->groups), order, nheavy, skip, ap, ks[0], ah,
+                                   (DevStatus*)(ah.ctr + 4), kgrid[0], s, &any))
+                return -1;
+            if (any)
+                out.ahead = ah;
+        }
         for (size_t b = 0; b < kind.size(); b++)
         {
             // a class on the wide instance has no wider one to hand groups to
@@ -1266,6 +1302,7 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
             AlignOut outw = out;
             outw.wide_list = nullptr;
             outw.nwide = nullptr;
+            outw.ahead = Ahead{};  // its places are those of another order
             if (launch_align_pairs(A.blk, B.blk, hkey, hdiag, P<uint2>(c->groups), wide_list, nwide, ap, scw, outw,
                                    P<unsigned>(c->queue), P<DevStatus>(c->status), c->agrid_w, s, 1))
                 return -1;
@@ -1561,7 +1598,8 @@ void gd_destroy(gd_context* c)
                       &c->okey0, &c->okey1, &c->oval0, &c->oval1, &c->olen, &c->las_raw, &c->las_off,
                       &c->las_rec, &c->las_out, &c->ascr_w, &c->wide, &c->ascr_d, &c->vf_rec, &c->vf_first,
                       &c->vf_trace, &c->vf_seg, &c->vf_list, &c->vf_diff, &c->vf_misc, &c->vf_scr, &c->lb_a, &c->lb_b,
-                      &c->lb_pka, &c->lb_pkb, &c->lb_in, &c->lb_out, &c->lb_tr};
+                      &c->lb_pka, &c->lb_pkb, &c->lb_in, &c->lb_out, &c->lb_tr,
+                      &c->ah_path, &c->ah_misc, &c->ah_trace};
     for (DevBuf* b : bufs)
         release(*b);
     for (HostBuf* h : {&c->h_rec, &c->h_tr})
