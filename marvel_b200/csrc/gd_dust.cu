@@ -186,8 +186,6 @@ __global__ void __launch_bounds__(64) k_dust_read(DevBlock blk, int W, double T,
     nout[r] = n;
 }
 
-constexpr int DUST_CHUNK = 1024;  // interval starts per chunk
-constexpr int DT = 128;           // chunks per block
 
 // Without -b: a chunk of a read per thread.  A chunk owns the intervals that start in its
 // DUST_CHUNK positions.  The window (wb, j] and the run (lb, j] at position j follow from the
@@ -195,21 +193,37 @@ constexpr int DT = 128;           // chunks per block
 // triplet is more frequent than the threshold allows (each step moves it just far enough).  A
 // candidate that starts at x is made, raised and tested at positions from x to x + W - 2 only, with
 // windows that reach back to x - W, against candidates that start at or behind x.  So a scan
-// begun 2W positions before the chunk has, from the chunk's first retirement on, exactly the
-// candidates of the whole read's scan.  The chunk's retired candidates come in order of their
+// begun W positions before the chunk, which makes candidates from the chunk's first start on
+// only, has the same candidates there as the whole read's scan.  The chunk's retired candidates come in order of their
 // starts and are merged as the reference merges them; k_dust_merge joins the chunks' lists,
 // which merges the same sequence in pieces.
 //
-// Bound by latency of the dependent steps, so the split is for warps in flight: one thread per
-// read (a 105 Mbp block of 10,020 reads) took 91 ms, its longest reads deciding; chunks give
-// 103,000 threads, 19 % of their steps spent on the starts.  Both counts of a triplet share
-// one shared-memory word ([triplet][thread], free of bank conflicts): the window's in the low
-// half, the run's in the high half.
+// One thread per read (a 105 Mbp block of 10,020 reads) took 91 ms, its longest reads deciding.
+// With chunks the bound is divergence: one step in ten or so walks the window from the run's start
+// down to its own (up to W - 2 places), and with the walk as an inner loop nearly every step of a
+// warp waited for some lane's (20 ms at any chunk size).  So a lane is either stepping or walking,
+// and every turn of the one loop takes each lane one step or one place further.  The walk counts
+// the triplets it meets on top of the run's in a field of its own, valid under the walk's tag,
+// so that nothing has to be walked back.  A triplet's counts share one shared-memory word
+// ([triplet][thread], free of bank conflicts): window, run, walk and tag, 8 bits each (a
+// window holds at most 126 triplets).  Triplets come from the 2-bit copy (any one-to-one code of
+// a triplet serves, so its bits stay as they are packed), and the walk compares the run's
+// integer sum with a table of the thresholds ceil(T n), which is the comparison of doubles it
+// stands for.  The worst chunks lie in tandem repeats, where every step walks: hence the short
+// chunks, for more warm-up elsewhere (the block takes 14.5 ms with chunks of 512, 12.1 with 256, 11.2
+// with 128, 12.0 with 64).
+constexpr int DUST_CHUNK = 128;  // interval starts per chunk
+constexpr int DT = 128;          // chunks per block
+
 __global__ void __launch_bounds__(DT) k_dust_chunks(DevBlock blk, int W, double T, int thr2,
                                                     const uint32_t* __restrict__ cfirst, unsigned nchunks, int* out,
                                                     int* __restrict__ ccount)
 {
     __shared__ unsigned cnt[64][DT];
+    __shared__ int thr[DUST_MAXW + 1];  // (double)s >= T * n  <=>  s >= thr[n], for whole s
+    for (int n = threadIdx.x; n <= DUST_MAXW; n += DT)
+        thr[n] = (int)fmin(ceil(__dmul_rn(T, (double)n)), 1e9);
+    __syncthreads();
     const unsigned g = blockIdx.x * DT + threadIdx.x;
     if (g >= nchunks)
         return;
@@ -224,19 +238,21 @@ __global__ void __launch_bounds__(DT) k_dust_chunks(DevBlock blk, int W, double 
     }
     const int r = lo;
     const int len = blk.rlen[r] - 2;
-    const uint8_t* b = blk.bases + blk.boff[r];
+    const uint32_t pk0 = PK_BIAS + (uint32_t)blk.boff[r];
+    auto trip = [&](int x) {  // the triplet at x
+        const uint32_t i = pk0 + (uint32_t)x;
+        return (int)(__funnelshift_r(__ldg(blk.pk + (i >> 4)), __ldg(blk.pk + (i >> 4) + 1), 2 * i) & 63u);
+    };
     const int b0 = (int)(g - cfirst[r]) * DUST_CHUNK, b1 = min(b0 + DUST_CHUNK, len);
     int* const list = out + blk.boff[r] + 4ll * r + b0;  // [begin, end] pairs, more than 3 apart
-    const int js = max(0, b0 - 2 * W), je = min(len, b1 + W - 2);
+    const int js = max(0, b0 - W), je = min(len, b1 + W - 2);
     unsigned* const my = &cnt[0][threadIdx.x];
     for (int e = 0; e < 64; e++)
         my[e * DT] = 0;
     DustCand cd[DUST_MAXW + 1];
     cd[0].beg = -2;
     cd[0].prev = cd[0].next = 0;
-    for (int i = 1; i <= W; i++)
-        cd[i].next = (i < W) ? i + 1 : -1;
-    int freel = 1, wb = js - 1, lb = js - 1, ws = 0, ls = 0;
+    int freel = 0, used = 0, wb = js - 1, lb = js - 1, ws = 0, ls = 0;
     int n = 0, mbeg = -2, mend = -2;  // the list and its open interval
     auto retire = [&](int beg, int end) {
         if (beg < b0 || beg >= b1)
@@ -255,74 +271,26 @@ __global__ void __launch_bounds__(DT) k_dust_chunks(DevBlock blk, int W, double 
             mend = c;
         }
     };
-    // the triplets entering and leaving roll with their positions
-    int cj = (b[js] << 2) | b[js + 1], cw = cj, cl = cj;
     int oldest = INT_MAX;  // start of the oldest candidate
     bool full = false;
-    for (int j = js; j < je; j++)
+    int j = js - 1;
+    // the walk: its next place, the last place before its end, sum, tag and place among the candidates
+    int x = 0, xend = 0, lw = 0, jp = 0, lp = 0;
+    unsigned tag = 0;
+    double ms = 0.;
+    while (true)
     {
-        cj = ((cj << 2) | b[j + 2]) & 63;
-        const int c = cj;
-        if (j - js > W - 3)
+        if (x > xend)
         {
-            wb++;
-            cw = ((cw << 2) | b[wb + 2]) & 63;
-            const unsigned v = my[cw * DT] - 1u;
-            my[cw * DT] = v;
-            ws -= (int)(v & 0xffffu);
-        }
-        if (lb < wb)
-        {
-            lb++;
-            cl = ((cl << 2) | b[lb + 2]) & 63;
-            const unsigned v = my[cl * DT] - 0x10000u;
-            my[cl * DT] = v;
-            ls -= (int)(v >> 16);
-        }
-        {
-            const unsigned v = my[c * DT];
-            ws += (int)(v & 0xffffu);
-            const int tr = (int)(v >> 16);
-            ls += tr;
-            my[c * DT] = v + 0x10001u;
-            if (tr >= thr2)
-                while (lb < j)
-                {
-                    lb++;
-                    cl = ((cl << 2) | b[lb + 2]) & 63;
-                    const unsigned u = my[cl * DT] - 0x10000u;
-                    my[cl * DT] = u;
-                    ls -= (int)(u >> 16);
-                    if (cl == c)
-                        break;
-                }
-        }
-        // retire the oldest candidate once its start has left the window
-        if (oldest <= wb)
-        {
-            const int t = cd[0].prev;
-            retire(cd[t].beg, cd[t].end);
-            const int q = cd[t].prev;
-            cd[0].prev = q;
-            cd[q].next = 0;
-            cd[t].next = freel;
-            freel = t;
-            oldest = q ? cd[q].beg : INT_MAX;
-        }
-        double lsq = (double)ls;
-        if ((double)ws <= __dmul_rn(lsq, T))
-            continue;
-        int jp = cd[0].next, lp = 0, x;
-        double ms = 0.;
-        for (x = lb; x > wb; x--)
-        {
-            const int d = dtrip(b, x);
+            // one place of the walk
+            const int d = trip(x);
             const unsigned v = my[d * DT];
-            ls += (int)(v >> 16);
-            my[d * DT] = v + 0x10000u;
-            lsq = (double)ls;
-            if (lsq >= __dmul_rn(T, (double)(j - x)))
+            const unsigned wk = (v >> 24) == tag ? (v >> 16) & 0xffu : 0u;
+            lw += (int)(((v >> 8) & 0xffu) + wk);
+            my[d * DT] = (v & 0xffffu) | ((wk + 1) << 16) | (tag << 24);
+            if (lw >= thr[j - x])
             {
+                const double lsq = (double)lw;
                 for (; cd[jp].beg >= x; lp = jp, jp = cd[jp].next)
                     if (cd[jp].score > ms)
                         ms = cd[jp].score;
@@ -336,13 +304,16 @@ __global__ void __launch_bounds__(DT) k_dust_chunks(DevBlock blk, int W, double 
                     }
                     else
                     {
-                        const int q = freel;
-                        if (q < 0)
+                        int q = freel;
+                        if (q)
+                            freel = cd[q].next;
+                        else if (used < W)
+                            q = ++used;
+                        else
                         {
                             full = true;  // candidate pool exhausted
                             break;
                         }
-                        freel = cd[q].next;
                         cd[q].beg = x;
                         cd[q].end = j;
                         cd[q].score = ms;
@@ -356,15 +327,70 @@ __global__ void __launch_bounds__(DT) k_dust_chunks(DevBlock blk, int W, double 
                     }
                 }
             }
+            x--;
         }
-        if (full)
-            break;
-        for (x++; x <= lb; x++)
+        else
         {
-            const int d = dtrip(b, x);
-            const unsigned v = my[d * DT] - 0x10000u;
-            my[d * DT] = v;
-            ls -= (int)(v >> 16);
+            // one step of the scan
+            if (++j >= je)
+                break;
+            const int c = trip(j);
+            if (j - js > W - 3)
+            {
+                const int d = trip(++wb);
+                const unsigned v = my[d * DT] - 1u;
+                my[d * DT] = v;
+                ws -= (int)(v & 0xffu);
+            }
+            if (lb < wb)
+            {
+                const int d = trip(++lb);
+                const unsigned v = my[d * DT] - 0x100u;
+                my[d * DT] = v;
+                ls -= (int)((v >> 8) & 0xffu);
+            }
+            const unsigned v = my[c * DT];
+            ws += (int)(v & 0xffu);
+            const int tr = (int)((v >> 8) & 0xffu);
+            ls += tr;
+            my[c * DT] = v + 0x101u;
+            if (tr >= thr2)
+                while (lb < j)
+                {
+                    const int d = trip(++lb);
+                    const unsigned u = my[d * DT] - 0x100u;
+                    my[d * DT] = u;
+                    ls -= (int)((u >> 8) & 0xffu);
+                    if (d == c)
+                        break;
+                }
+            // retire the oldest candidate once its start has left the window
+            if (oldest <= wb)
+            {
+                const int t = cd[0].prev;
+                retire(cd[t].beg, cd[t].end);
+                const int q = cd[t].prev;
+                cd[0].prev = q;
+                cd[q].next = 0;
+                cd[t].next = freel;
+                freel = t;
+                oldest = q ? cd[q].beg : INT_MAX;
+            }
+            xend = x = max(wb, b0 - 1);
+            if ((double)ws > __dmul_rn((double)ls, T))
+            {
+                x = lb;
+                lw = ls;
+                jp = cd[0].next;
+                lp = 0;
+                ms = 0.;
+                if (++tag == 256)  // the tags are used up: clear them
+                {
+                    tag = 1;
+                    for (int e = 0; e < 64; e++)
+                        my[e * DT] &= 0xffffu;
+                }
+            }
         }
     }
     for (int t = cd[0].prev; t != 0 && !full; t = cd[t].prev)

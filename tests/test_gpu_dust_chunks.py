@@ -7,7 +7,7 @@ from marvel_b200 import dazzdb
 
 pytestmark = pytest.mark.gpu
 
-CHUNK = 1024  # interval starts per chunk (gd_dust.cu)
+CHUNK = 128  # interval starts per chunk (gd_dust.cu)
 
 
 def block(rng, window):
