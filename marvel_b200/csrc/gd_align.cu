@@ -309,6 +309,16 @@ __device__ __forceinline__ int snake_pk(const bool FWD, const uint32_t* __restri
     }
 }
 
+// snake_pk out of line for the 0-wave: (y, bend | aend << 1).  The pair kernel's code is near the size
+// its instruction cache holds (in line, the 121 Mbp block's aligner took 185.5 ms instead of 183).
+__device__ __noinline__ int2 snake_begin(const bool FWD, const uint32_t* __restrict__ apk, uint32_t ag,
+                                         const uint32_t* __restrict__ bpk, uint32_t bg, int y, int k, int alen, int blen)
+{
+    bool bend, aend;
+    y = snake_pk(FWD, apk, ag, bpk, bg, y, k, alen, blen, bend, aend);
+    return make_int2(y, (bend ? 1 : 0) | (aend ? 2 : 0));
+}
+
 // The trim test of forward_wave/reverse_wave (align.c:884-896): the newest 15 columns are
 // suffix-positive and so are the newest 30 (TABLE / SCORE built by set_table, align.c:196-210).
 __device__ __forceinline__ bool trim_ok(unsigned long long b, const int16_t* table, const int16_t* score)
@@ -402,8 +412,15 @@ __device__ __forceinline__ void wave_begin(const bool FWD, WarpCtx<RG>& w, WaveV
             hb = peb_one(w, npeb, -1, k, 0, y);
         }
         bool bend, aend;
-        y = PK ? snake_pk(FWD, apk, ag, bpk, bg, y, k, alen, blen, bend, aend)
-               : snake(FWD, aseq0, bseq0, y, k, blen + 16, bend, aend);
+        if (PK)
+        {
+            const int2 f = snake_begin(FWD, apk, ag, bpk, bg, y, k, alen, blen);
+            y = f.x;
+            bend = f.y & 1;
+            aend = f.y & 2;
+        }
+        else
+            y = snake(FWD, aseq0, bseq0, y, k, blen + 16, bend, aend);
         if (bend)
         {
             more = 0;
@@ -940,7 +957,8 @@ __device__ __forceinline__ bool wave_step(const bool FWD, WarpCtx<RG>& w, WaveVa
 // carries per diagonal are never ahead of or behind that), which the predecessor's position
 // gives, and so no pebble is read back for its mark either.  On a 21 Mbp block (25 M waves per
 // orientation) the kernel issues 6.6 G warp instructions instead of 8.2 G and takes 7.9 ms
-// instead of 9.4; it stays bound by issue (76 % of the slots) and the dependent chain of a wave.
+// instead of 9.4; with the extension's first 16 bases in line and fewer branches 6.4 G and 7.6 ms.
+// It stays bound by issue (76 % of the slots) and the dependent chain of a wave.
 //
 // Runs waves until the wave loop ends (false; or an error in w.err) or the band or anything
 // unusual asks for wave_step (true; the state is then in the ring).
@@ -1020,15 +1038,25 @@ __device__ __forceinline__ bool wave_regs(WarpCtx<RG>& w, WaveVars& wvars, const
         if (valid)
         {
             const int y0 = y, x0 = y + k;
-            y = snake_pk(FWD, apk, ag, bpk, bg, y, k, alen, blen, bend, aend);
-            const int L = FWD ? y - y0 : y0 - y;
-            if ((unsigned)L < 31u)
+            // the first 16 bases of snake_pk in line; the rare longer match in its loop
+            const int eb = FWD ? blen - y0 : y0, ea = FWD ? alen - x0 : x0, en = min(ea, eb);
+            const uint32_t sb = FWD ? bg + y0 : bg + y0 - 16, sa = FWD ? ag + x0 : ag + x0 - 16;
+            const uint32_t wb = __funnelshift_r(__ldg(bpk + (sb >> 4)), __ldg(bpk + (sb >> 4) + 1), 2 * sb);
+            const uint32_t wa = __funnelshift_r(__ldg(apk + (sa >> 4)), __ldg(apk + (sa >> 4) + 1), 2 * sa);
+            const uint32_t dd = wa ^ wb;
+            const int s = min((FWD ? __clz((int)__brev(dd)) : __clz((int)dd)) >> 1, en);
+            if ((unsigned)s < 16u)
             {
-                t1 = __funnelshift_l(t0, t1, L + 1);
-                t0 = (t0 << (L + 1)) | ((1u << L) - 1u);
+                t1 = __funnelshift_l(t0, t1, s + 1);
+                t0 = (t0 << (s + 1)) | ((1u << s) - 1u);
+                y = FWD ? y0 + s : y0 - s;
+                bend = s == eb;
+                aend = (s == ea) & !bend;
             }
             else
             {
+                y = snake_pk(FWD, apk, ag, bpk, bg, y0, k, alen, blen, bend, aend);
+                const int L = FWD ? y - y0 : y0 - y;
                 unsigned long long b = (((unsigned long long)t1 << 32) | t0) << 1;
                 b = (L >= 61) ? ~0ull : ((b << L) | ((1ull << L) - 1ull));
                 t0 = (uint32_t)b;
@@ -1090,8 +1118,14 @@ __device__ __forceinline__ bool wave_regs(WarpCtx<RG>& w, WaveVars& wvars, const
         // the best point (align.c:880-897): the first diagonal in scan order with the largest V,
         // value and place in one reduction
         const int wbest = FWD ? besta : -besta;
-        const bool q1 = (key >> 5) > wbest && __popc(t0) + __popc(t1 & (uint32_t)(MASK61 >> 32)) >= PATH_AVE;
-        const bool q2 = q1 && trim_ok(t0, P.table, P.score);
+        const bool q1 = ((key >> 5) > wbest) & (__popc(t0) + __popc(t1 & (uint32_t)(MASK61 >> 32)) >= PATH_AVE);
+        bool q2 = false;
+        if (q1)
+        {
+            const int lo15 = (int)(t0 & TRIM_MASK), hi15 = (int)((t0 >> TRIM_LEN) & TRIM_MASK);
+            const int tl = __ldg(P.table + lo15), th = __ldg(P.table + hi15), sl = __ldg(P.score + lo15);
+            q2 = (tl >= 0) & (th + sl >= 0);
+        }
         const int kmax = __reduce_max_sync(GD_FULL, key);
         const bool better = (kmax >> 5) > wbest;
         const int jm = 31 - (kmax & 31);

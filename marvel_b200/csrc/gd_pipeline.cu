@@ -2591,14 +2591,20 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     }
     if (nseeds <= 0)
         return 0;
-    if (alen_total + 256 > 0xffffffffll || blen_total + 256 > 0xffffffffll)
-    {
-        gd_set_error("Local_Alignment batch: sequences beyond this build's 32-bit base index");
-        return -1;
-    }
+    // the waves read 2-bit copies, which end at the lengths, where every read has its 4s at just
+    // those ends (as blocks have them) and the copies' 32-bit index reaches; else the bytes, whose
+    // 4s stop them
+    bool packed = alen_total + 256 <= 0xffffffffll && blen_total + 256 <= 0xffffffffll;
+    auto ends = [](const uint8_t* s, int64_t total, int64_t off, int32_t len) {
+        auto four = [&](int64_t i) { return i < 0 || i >= total || s[i] == 4; };
+        return off >= 0 && four(off - 1) && four(off + len);
+    };
     int maxlen = 0;
     for (int i = 0; i < nseeds; i++)
+    {
         maxlen = std::max(maxlen, std::max(alen[i], blen[i]));
+        packed = packed && ends(abases, alen_total, aoff[i], alen[i]) && ends(bbases, blen_total, boff[i], blen[i]);
+    }
     AlignParams ap{};
     ap.tspace = c->tspace;
     ap.ave_path = c->ave_path;
@@ -2644,11 +2650,11 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     GD_CUDA(cudaMemcpyAsync(d_dg, diag, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_an, anti, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemsetAsync(c->lb_out.p, 0, n8 + 12 * n4 + 64, s));
-    if (launch_pack2(P<uint8_t>(c->lb_a), alen_total + 128, P<uint32_t>(c->lb_pka), wa, s) ||
-        launch_pack2(P<uint8_t>(c->lb_b), blen_total + 128, P<uint32_t>(c->lb_pkb), wb, s) ||
+    if ((packed && (launch_pack2(P<uint8_t>(c->lb_a), alen_total + 128, P<uint32_t>(c->lb_pka), wa, s) ||
+                    launch_pack2(P<uint8_t>(c->lb_b), blen_total + 128, P<uint32_t>(c->lb_pkb), wb, s))) ||
         launch_la_batch(P<uint8_t>(c->lb_a) + 64, d_ao, d_al, P<uint8_t>(c->lb_b) + 64, d_bo, d_bl, d_dg, d_an, nseeds,
-                        ap, sc, d_out, P<uint16_t>(c->lb_tr), trstride, d_cells, d_st, s, P<uint32_t>(c->lb_pka), 64,
-                        P<uint32_t>(c->lb_pkb), 64))
+                        ap, sc, d_out, P<uint16_t>(c->lb_tr), trstride, d_cells, d_st, s,
+                        packed ? P<uint32_t>(c->lb_pka) : nullptr, 64, packed ? P<uint32_t>(c->lb_pkb) : nullptr, 64))
         return -1;
     DevStatus st;
     GD_CUDA(cudaMemcpyAsync(&st, d_st, sizeof st, cudaMemcpyDeviceToHost, s));

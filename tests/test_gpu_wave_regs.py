@@ -79,3 +79,23 @@ def test_waves_match_oracle(ts, comp):
         assert (tr[n, :o[5]] == at).all() and (tr[n, half:half + o[11]] == bt).all()
         assert cells[n] == oc
     ctx.close()
+
+
+def test_batch_of_a_longer_read_than_its_length_reads_bytes():
+    """A length that ends before the read's 4: the byte waves run on to the 4, as they always have."""
+    import marvel_b200 as mb
+    import oracle
+    rng = np.random.default_rng(3)
+    s = rng.integers(0, 4, 3000, dtype=np.uint8)
+    a, b = mutate(rng, s, 0.1), mutate(rng, s, 0.1)
+    freq = np.full(4, .25, np.float32)
+    ctx = mb.Context()
+    ctx.new_align_spec(0.70, 100, freq)
+    four = np.array([4], np.uint8)
+    abuf, bbuf = np.concatenate([four, a, four]), np.concatenate([four, b, four])
+    one = np.ones(1, np.int64)
+    o, at, bt, oc = oracle.local_alignment(abuf, bbuf, 0, 0, 0, oracle.make_params(freq))
+    out, tr, cells = ctx.local_alignment_batch(abuf, one, [a.size - 1], bbuf, one, [b.size], [0], [0], 0)
+    assert out[0, :7].tolist() == o[:7].tolist() and cells[0] == oc
+    assert (tr[0, :o[5]] == at).all()
+    ctx.close()
