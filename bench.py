@@ -402,9 +402,9 @@ def run_gpu(args):
                          "traffic_source": "bytes per launch: dram read+write per wave cell of the cfg1 ncu capture "
                                            "(profiles/k_align_pairs_cfg1.md) x this launch's cells",
                          "peak_source": "derived: 148 SM x 128 lanes/clk x median SM clock under load",
-                         "issue_slots_busy": 0.781,
-                         "issue_source": "smsp__issue_active of the cfg1 ncu capture (profiles/k_align_pairs_cfg1.md): "
-                                         "the kernel issues on 78 % of cycles; a wave is ~11 diagonals wide, so a "
+                         "issue_slots_busy": 0.765,
+                         "issue_source": "smsp__issue_active of the 21 Mbp ncu capture (profiles/k_align_pairs_regs_21mbp.md): "
+                                         "the kernel issues on 76 % of cycles; a wave is ~11 diagonals wide, so a "
                                          "warp instruction carries about a third of a warp of cells"},
             "roofline_filter": {"bound": "hbm", "kernel": "k-mer index (extract + 4 LSD passes)",
                                 "achieved": round(idx_bytes / (idx_ms / 1e3) / 1e9, 1),
