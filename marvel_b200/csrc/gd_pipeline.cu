@@ -2578,6 +2578,11 @@ int gd_get_stats(gd_context* c, gd_stats* st)
     return 0;
 }
 
+// 4s before and after the batch's sequences.  The byte waves stop at 4s, but where a length runs past
+// its read's 4 they go on until the band has fallen TRIM_MLAG anti-diagonals behind, up to a few hundred
+// bases beyond the last one
+constexpr int64_t LA_PAD = 512;
+
 int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_total, const uint8_t* bbases,
                              int64_t blen_total, const int64_t* aoff, const int32_t* alen, const int64_t* boff,
                              const int32_t* blen, const int32_t* diag, const int32_t* anti, int nseeds, int comp,
@@ -2591,19 +2596,29 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     }
     if (nseeds <= 0)
         return 0;
-    // the waves read 2-bit copies, which end at the lengths, where every read has its 4s at just
-    // those ends (as blocks have them) and the copies' 32-bit index reaches; else the bytes, whose
-    // 4s stop them
-    bool packed = alen_total + 256 <= 0xffffffffll && blen_total + 256 <= 0xffffffffll;
-    auto ends = [](const uint8_t* s, int64_t total, int64_t off, int32_t len) {
+    // the waves read 2-bit copies, which end at the lengths, where every read lies in its buffer
+    // with its 4s at just its ends (as blocks have them), every seed in its reads, and the
+    // copies' 32-bit index reaches; else the bytes, whose 4s stop them
+    const int64_t abytes = alen_total + 2 * LA_PAD, bbytes = blen_total + 2 * LA_PAD;
+    bool packed = abytes <= 0xffffffffll && bbytes <= 0xffffffffll;
+    auto whole = [](const uint8_t* s, int64_t total, int64_t off, int32_t len, int64_t at) {
         auto four = [&](int64_t i) { return i < 0 || i >= total || s[i] == 4; };
-        return off >= 0 && four(off - 1) && four(off + len);
+        return off >= 0 && off <= total && len >= 0 && len <= total - off && at >= 0 && at <= len && four(off - 1) &&
+               four(off + len);
     };
     int maxlen = 0;
     for (int i = 0; i < nseeds; i++)
     {
         maxlen = std::max(maxlen, std::max(alen[i], blen[i]));
-        packed = packed && ends(abases, alen_total, aoff[i], alen[i]) && ends(bbases, blen_total, boff[i], blen[i]);
+        const int64_t y = ((int64_t)anti[i] - diag[i]) >> 1, x = y + diag[i];
+        for (const int64_t out : {-(aoff[i] + x), aoff[i] + x - alen_total, -(boff[i] + y), boff[i] + y - blen_total})
+            if (out > 64)  // the bytes beyond are nobody's; a seed that begins in the margin ends at once
+            {
+                gd_set_error("Local_Alignment batch: seed %d begins outside the sequences", i);
+                return -1;
+            }
+        packed = packed && whole(abases, alen_total, aoff[i], alen[i], x) &&
+                 whole(bbases, blen_total, boff[i], blen[i], y);
     }
     AlignParams ap{};
     ap.tspace = c->tspace;
@@ -2624,8 +2639,8 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     // the context keeps these buffers (the scratch is the pair aligner's); the call's own cudaMalloc
     // and cudaFree of 2 GB took most of its time
     const size_t n8 = (size_t)nseeds * 8, n4 = (size_t)nseeds * 4;
-    const int64_t wa = (alen_total + 128 + 15) / 16 + 1, wb = (blen_total + 128 + 15) / 16 + 1;
-    if (ensure(c->lb_a, alen_total + 128) || ensure(c->lb_b, blen_total + 128) || ensure(c->lb_pka, wa * 4) ||
+    const int64_t wa = (abytes + 15) / 16 + 1, wb = (bbytes + 15) / 16 + 1;
+    if (ensure(c->lb_a, abytes) || ensure(c->lb_b, bbytes) || ensure(c->lb_pka, wa * 4) ||
         ensure(c->lb_pkb, wb * 4) || ensure(c->lb_in, 2 * n8 + 4 * n4) || ensure(c->lb_out, n8 + 12 * n4 + 64) ||
         ensure(c->lb_tr, (size_t)nseeds * trstride * 2) ||
         ensure(c->ascr, align_scratch_bytes(nwarps, c->pcap, ptscap, 4, 4, 4)))
@@ -2638,10 +2653,10 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     int64_t* d_cells = (int64_t*)(P<char>(c->lb_out) + 64);
     int32_t* d_out = (int32_t*)(d_cells + nseeds);
     // sequences: caller buffers hold [4, read, 4, read, ...] with offsets relative to index 0
-    GD_CUDA(cudaMemsetAsync(c->lb_a.p, 4, alen_total + 128, s));
-    GD_CUDA(cudaMemsetAsync(c->lb_b.p, 4, blen_total + 128, s));
-    if (staged_copy(c->stage, P<uint8_t>(c->lb_a) + 64, (void*)abases, alen_total, true, s) ||
-        staged_copy(c->stage, P<uint8_t>(c->lb_b) + 64, (void*)bbases, blen_total, true, s))
+    GD_CUDA(cudaMemsetAsync(c->lb_a.p, 4, abytes, s));
+    GD_CUDA(cudaMemsetAsync(c->lb_b.p, 4, bbytes, s));
+    if (staged_copy(c->stage, P<uint8_t>(c->lb_a) + LA_PAD, (void*)abases, alen_total, true, s) ||
+        staged_copy(c->stage, P<uint8_t>(c->lb_b) + LA_PAD, (void*)bbases, blen_total, true, s))
         return -1;
     GD_CUDA(cudaMemcpyAsync(d_ao, aoff, n8, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_bo, boff, n8, cudaMemcpyHostToDevice, s));
@@ -2650,11 +2665,12 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     GD_CUDA(cudaMemcpyAsync(d_dg, diag, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_an, anti, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemsetAsync(c->lb_out.p, 0, n8 + 12 * n4 + 64, s));
-    if ((packed && (launch_pack2(P<uint8_t>(c->lb_a), alen_total + 128, P<uint32_t>(c->lb_pka), wa, s) ||
-                    launch_pack2(P<uint8_t>(c->lb_b), blen_total + 128, P<uint32_t>(c->lb_pkb), wb, s))) ||
-        launch_la_batch(P<uint8_t>(c->lb_a) + 64, d_ao, d_al, P<uint8_t>(c->lb_b) + 64, d_bo, d_bl, d_dg, d_an, nseeds,
-                        ap, sc, d_out, P<uint16_t>(c->lb_tr), trstride, d_cells, d_st, s,
-                        packed ? P<uint32_t>(c->lb_pka) : nullptr, 64, packed ? P<uint32_t>(c->lb_pkb) : nullptr, 64))
+    if ((packed && (launch_pack2(P<uint8_t>(c->lb_a), abytes, P<uint32_t>(c->lb_pka), wa, s) ||
+                    launch_pack2(P<uint8_t>(c->lb_b), bbytes, P<uint32_t>(c->lb_pkb), wb, s))) ||
+        launch_la_batch(P<uint8_t>(c->lb_a) + LA_PAD, d_ao, d_al, P<uint8_t>(c->lb_b) + LA_PAD, d_bo, d_bl, d_dg, d_an,
+                        nseeds, ap, sc, d_out, P<uint16_t>(c->lb_tr), trstride, d_cells, d_st, s,
+                        packed ? P<uint32_t>(c->lb_pka) : nullptr, LA_PAD, packed ? P<uint32_t>(c->lb_pkb) : nullptr,
+                        LA_PAD))
         return -1;
     DevStatus st;
     GD_CUDA(cudaMemcpyAsync(&st, d_st, sizeof st, cudaMemcpyDeviceToHost, s));
