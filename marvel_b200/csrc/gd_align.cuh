@@ -145,6 +145,11 @@ int launch_align_ahead(const DevBlock& A, const DevBlock& B, const uint64_t* hke
                        const uint2* groups, const uint32_t* order, unsigned nheavy, const uint8_t* skip, AlignParams p,
                        AlignScratch sc, Ahead ah, DevStatus* st, int grid, cudaStream_t s, bool* any);
 
+// *odd (preset 0) becomes 1 when a seed's reads hold anything but bases 0 to 3 between 4s.  The reads lie
+// in their buffers, which are 16-byte aligned with a margin on either side.
+int launch_la_plain(const uint8_t* aseq_base, const int64_t* aoff, const int32_t* alen, const uint8_t* bseq_base,
+                    const int64_t* boff, const int32_t* blen, int nseeds, unsigned* odd, cudaStream_t s);
+
 // One Local_Alignment per seed (for parity tests of the wave alone).  out12 per seed:
 // A-path {abpos,bbpos,aepos,bepos,diffs,tlen}, B-path the same; traces at
 // tr + seed * trstride (A) and tr + seed * trstride + trstride/2 (B).  With the buffers' 2-bit copies

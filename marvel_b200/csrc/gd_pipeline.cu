@@ -2597,14 +2597,12 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     if (nseeds <= 0)
         return 0;
     // the waves read 2-bit copies, which end at the lengths, where every read lies in its buffer
-    // with its 4s at just its ends (as blocks have them), every seed in its reads, and the
-    // copies' 32-bit index reaches; else the bytes, whose 4s stop them
+    // with 4s at just its ends (as blocks have them; the bytes are looked at on the device), every
+    // seed in its reads, and the copies' 32-bit index reaches; else the bytes, whose 4s stop them
     const int64_t abytes = alen_total + 2 * LA_PAD, bbytes = blen_total + 2 * LA_PAD;
     bool packed = abytes <= 0xffffffffll && bbytes <= 0xffffffffll;
-    auto whole = [](const uint8_t* s, int64_t total, int64_t off, int32_t len, int64_t at) {
-        auto four = [&](int64_t i) { return i < 0 || i >= total || s[i] == 4; };
-        return off >= 0 && off <= total && len >= 0 && len <= total - off && at >= 0 && at <= len && four(off - 1) &&
-               four(off + len);
+    auto whole = [](int64_t total, int64_t off, int32_t len, int64_t at) {
+        return off >= 0 && off <= total && len >= 0 && len <= total - off && at >= 0 && at <= len;
     };
     int maxlen = 0;
     for (int i = 0; i < nseeds; i++)
@@ -2617,8 +2615,7 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
                 gd_set_error("Local_Alignment batch: seed %d begins outside the sequences", i);
                 return -1;
             }
-        packed = packed && whole(abases, alen_total, aoff[i], alen[i], x) &&
-                 whole(bbases, blen_total, boff[i], blen[i], y);
+        packed = packed && whole(alen_total, aoff[i], alen[i], x) && whole(blen_total, boff[i], blen[i], y);
     }
     AlignParams ap{};
     ap.tspace = c->tspace;
@@ -2665,6 +2662,16 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     GD_CUDA(cudaMemcpyAsync(d_dg, diag, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_an, anti, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemsetAsync(c->lb_out.p, 0, n8 + 12 * n4 + 64, s));
+    if (packed)
+    {
+        unsigned odd = 0, *d_odd = (unsigned*)(d_st + 1);
+        if (launch_la_plain(P<uint8_t>(c->lb_a) + LA_PAD, d_ao, d_al, P<uint8_t>(c->lb_b) + LA_PAD, d_bo, d_bl, nseeds,
+                            d_odd, s))
+            return -1;
+        GD_CUDA(cudaMemcpyAsync(&odd, d_odd, 4, cudaMemcpyDeviceToHost, s));
+        GD_CUDA(cudaStreamSynchronize(s));
+        packed = !odd;
+    }
     if ((packed && (launch_pack2(P<uint8_t>(c->lb_a), abytes, P<uint32_t>(c->lb_pka), wa, s) ||
                     launch_pack2(P<uint8_t>(c->lb_b), bbytes, P<uint32_t>(c->lb_pkb), wb, s))) ||
         launch_la_batch(P<uint8_t>(c->lb_a) + LA_PAD, d_ao, d_al, P<uint8_t>(c->lb_b) + LA_PAD, d_bo, d_bl, d_dg, d_an,

@@ -88,6 +88,33 @@ def test_length_past_the_sequences(ctx, over, comp):
                   [0, 0, 0], [0, 1600, 3000], comp)
 
 
+@pytest.mark.parametrize("comp", [0, 1])
+@pytest.mark.parametrize("at", [0, 1, 7, 511, 1600, -2, -1])
+@pytest.mark.parametrize("value", [4, 5, 255])
+def test_byte_beyond_3_inside_a_read(ctx, value, at, comp):
+    """A 4 inside a read ends it there; other bytes match nothing but themselves.  In A, in B, in both."""
+    rng = np.random.default_rng(at % 97 + comp)
+    s = rng.integers(0, 4, 3000, dtype=np.uint8)
+    abuf, aoff, alen = joined([noisy(rng, s), noisy(rng, s)])
+    bbuf, boff, blen = joined([noisy(rng, s), noisy(rng, s)])
+    for buf, off, n in ((abuf, aoff, alen), (bbuf, boff, blen)):
+        buf[off[1] + at % n[1]] = value
+    i, j = np.array([1, 0, 1, 0]), np.array([0, 1, 1, 0])
+    same_as_bytes(ctx, abuf, aoff[i], alen[i], bbuf, boff[j], blen[j], [0, 2, -3, 1], [200, 1400, 2901, 3001], comp)
+
+
+@pytest.mark.parametrize("comp", [0, 1])
+def test_length_over_a_separator(ctx, comp):
+    """Lengths that take the 4 behind a read with them, or the read behind that too."""
+    rng = np.random.default_rng(40 + comp)
+    s = rng.integers(0, 4, 3000, dtype=np.uint8)
+    abuf, aoff, alen = joined([noisy(rng, s[:1500]), noisy(rng, s[1500:])])
+    bbuf, boff, blen = joined([noisy(rng, s), noisy(rng, s)])
+    both = alen[0] + 1 + alen[1]
+    same_as_bytes(ctx, abuf, aoff[[0, 0, 1]], np.array([alen[0] + 1, both, alen[1] + 1]), bbuf, boff[[0, 1, 1]],
+                  np.array([blen[0], blen[1] + 1, blen[1] + 1]), [0, 0, 0], [400, 400, 800], comp)
+
+
 def test_seed_outside_its_reads(ctx):
     """Positions beyond a read's ends but within its buffer, whose bytes the waves then read."""
     rng = np.random.default_rng(5)
