@@ -2662,6 +2662,8 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     GD_CUDA(cudaMemcpyAsync(d_dg, diag, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_an, anti, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemsetAsync(c->lb_out.p, 0, n8 + 12 * n4 + 64, s));
+    // the rows go to the caller whole: zeros behind a trace, not an earlier call's
+    GD_CUDA(cudaMemsetAsync(c->lb_tr.p, 0, (size_t)nseeds * trstride * 2, s));
     if (packed)
     {
         unsigned odd = 0, *d_odd = (unsigned*)(d_st + 1);

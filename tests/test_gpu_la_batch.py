@@ -131,3 +131,24 @@ def test_seed_outside_the_sequences_is_refused(ctx):
     for o, x, y in ((1, 600, 0), (1, 0, 600), (1, -90, 0), (1, 0, -90), (-200, 0, 0), (5000, 0, 0), (1, 1 << 29, 0)):
         with pytest.raises(mb.GpuError, match="outside the sequences"):
             ctx.local_alignment_batch(buf, [o], n, buf, [o], n, [x - y], [x + y], 0)
+
+
+def test_results_do_not_depend_on_earlier_calls(ctx):
+    """Whole trace rows, the part behind the trace included."""
+    import marvel_b200 as mb
+    rng = np.random.default_rng(8)
+    s = rng.integers(0, 4, 4000, dtype=np.uint8)
+    buf, off, n = joined([noisy(rng, s), noisy(rng, s)])
+    first = (buf, off[[0, 0]], n[[0, 0]], buf.copy(), off[[1, 1]], n[[1, 1]], [0, 0], [3000, 5000], 0)
+    second = (buf, off[[0, 0]], n[[0, 0]], buf.copy(), off[[1, 1]], n[[1, 1]], [900, -900], [3100, 5000], 0)
+    ctx.local_alignment_batch(*first)
+    got = ctx.local_alignment_batch(*second)
+    fresh = mb.Context()
+    fresh.new_align_spec(0.70, 100, np.full(4, .25, np.float32))
+    want = fresh.local_alignment_batch(*second)
+    fresh.close()
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
+    half = got[1].shape[1] // 2
+    for o, row in zip(*got[:2]):
+        assert not row[o[5]:half].any() and not row[half + o[11]:].any()
