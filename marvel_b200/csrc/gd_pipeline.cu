@@ -12,6 +12,7 @@
 #include <cstdarg>
 #include <cstring>
 #include <functional>
+#include <initializer_list>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -261,6 +262,7 @@ struct Slot
     int64_t totlen = 0, nslots = 0;
     int64_t nmask = 0;  // ints of mask interval data
     int has_mask = 0, loaded = 0;
+    int plain = -1;  // reads of bases 0 to 3 only; -1: not looked at yet
     DevBuf code, read, rpos;
     int64_t nk = -1;
     std::vector<int32_t> hrlen;
@@ -1747,6 +1749,7 @@ int gd_load_block(gd_context* c, int slot, const gd_block* b)
     s.nslots = nb - (int64_t)c->kmer * b->nreads;
     s.hrlen.assign(b->rlen, b->rlen + b->nreads);
     s.loaded = 1;
+    s.plain = -1;
     s.nk = -1;
     GD_CUDA(cudaStreamSynchronize(c->s));
     return 0;
@@ -1812,6 +1815,7 @@ int gd_complement_block(gd_context* c, int src, int dst)
     D.nslots = S.nslots;
     D.hrlen = S.hrlen;
     D.loaded = 1;
+    D.plain = S.plain;
     D.nk = -1;
     GD_CUDA(cudaStreamSynchronize(c->s));
     return 0;
@@ -2402,6 +2406,31 @@ int gd_write_overlap_buffer(gd_context* c, int run_id, const char* ablock, const
     return write_las(c, p2, j, nsrt);
 }
 
+// whether all bases of the slots' blocks are 0 to 3 (the 2-bit copies hold no others): 1, 0, or -1 on failure
+static int slots_plain(gd_context* c, std::initializer_list<Slot*> slots)
+{
+    unsigned odd[3], n = 0;
+    Slot* unknown[3];
+    if (ensure(c->vf_misc, 64))
+        return -1;
+    GD_CUDA(cudaMemsetAsync(c->vf_misc.p, 0, sizeof odd, c->s));
+    for (Slot* s : slots)
+        if (s->loaded && s->plain < 0 && std::find(unknown, unknown + n, s) == unknown + n)
+        {
+            if (gd::launch_block_plain(s->blk, P<unsigned>(c->vf_misc) + n, c->s))
+                return -1;
+            unknown[n++] = s;
+        }
+    if (n)
+    {
+        GD_CUDA(cudaMemcpyAsync(odd, c->vf_misc.p, sizeof odd, cudaMemcpyDeviceToHost, c->s));
+        GD_CUDA(cudaStreamSynchronize(c->s));
+    }
+    for (unsigned i = 0; i < n; i++)
+        unknown[i]->plain = !odd[i];
+    return std::all_of(slots.begin(), slots.end(), [](Slot* s) { return !s->loaded || s->plain; });
+}
+
 int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const gd_overlap* recs, const uint8_t* trace,
                          int64_t n, int32_t* diffs_out)
 {
@@ -2459,6 +2488,9 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
         tlo = thi = 0;
     const DevBlock& Cb = Cc.loaded ? Cc.blk : B.blk;
     cudaStream_t s = c->s;
+    const int plain = slots_plain(c, {&A, &B, &Cc});
+    if (plain < 0)
+        return -1;
     if (ensure(c->vf_rec, (size_t)n * sizeof(OutRec)) || ensure(c->vf_first, (size_t)(n + 1) * 8) ||
         ensure(c->vf_trace, (size_t)(thi - tlo) + 16) || ensure(c->vf_seg, (size_t)nseg * sizeof(Segment)) ||
         ensure(c->vf_list, (size_t)nseg * 4) || ensure(c->vf_diff, (size_t)n * 4) || ensure(c->vf_misc, 64))
@@ -2479,7 +2511,7 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
     if (launch_trace_segments(P<OutRec>(c->vf_rec), n, P<int64_t>(c->vf_first), P<uint8_t>(c->vf_trace), tlo, TS, tbytes,
                               A.blk.ufirst, B.blk.ufirst, P<Segment>(c->vf_seg), misc + 1, dst, s) ||
         launch_trace_pts(A.blk, B.blk, Cb, P<Segment>(c->vf_seg), nseg, P<int>(c->vf_diff), P<unsigned>(c->vf_list), misc,
-                         s))
+                         plain, s))
         return -1;
     unsigned h[8];
     GD_CUDA(cudaMemcpyAsync(h, misc, sizeof h, cudaMemcpyDeviceToHost, s));
