@@ -7,7 +7,8 @@
  * success and -1 on failure, with the message in gd_last_error(); nothing exits the
  * process (the reference calls exit(1) instead, dalign/filter.c:2135-2145).
  *
- * One context = one GPU (the device current at gd_create) and one host thread.
+ * One context = one GPU (the device current at gd_create) and one host thread at a time:
+ * calls on one context from several threads take turns.
  */
 #ifndef GPUDALIGN_H
 #define GPUDALIGN_H

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <functional>
 #include <initializer_list>
+#include <mutex>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -280,6 +281,10 @@ int bits_for(int64_t maxval)
 
 struct gd_context
 {
+    // calls from several threads take turns: buffers, staging and scratch outlive a call and are
+    // shared by all of them (a threaded caller of the reference's Local_Alignment has one spec,
+    // and so one context, for all its threads)
+    std::recursive_mutex turn;
     cudaStream_t s = nullptr;
     int kmer = 14, binshift = 6, suppress = 0, hitmin = 35;
     double ave_corr = .70;
@@ -338,6 +343,8 @@ struct gd_context
     std::vector<float> tri_hfeat;
     std::vector<uint32_t> tri_hrec, tri_hcells;
 };
+
+using Turn = std::lock_guard<std::recursive_mutex>;
 
 // ----------------------------------------------------------------------------------------
 // align spec: trim tables (set_table / New_Align_Spec, dalign/align.c:196-279)
@@ -1646,6 +1653,7 @@ int gd_set_filter_params(gd_context* c, int kmer, int binshift, int suppress, in
 int gd_new_align_spec(gd_context* c, double ave_corr, int trace_space, const float freq[4], int symmetric,
                       int only_identity, int no_trace_points)
 {
+    Turn turn(c->turn);
     if (trace_space <= 0)
     {
         gd_set_error("invalid trace spacing of (%d)", trace_space);
@@ -1675,6 +1683,7 @@ static int pack_slot(gd_context* c, Slot& s, int64_t nbytes);
 
 int gd_load_block(gd_context* c, int slot, const gd_block* b)
 {
+    Turn turn(c->turn);
     if (slot < 0 || slot > 2)
     {
         gd_set_error("slot %d out of range", slot);
@@ -1773,6 +1782,7 @@ static int pack_slot(gd_context* c, Slot& s, int64_t nbytes)
 
 int gd_complement_block(gd_context* c, int src, int dst)
 {
+    Turn turn(c->turn);
     if (src < 0 || src > 2 || dst < 0 || dst > 2 || src == dst || !c->slot[src].loaded)
     {
         gd_set_error("bad complement slots %d -> %d", src, dst);
@@ -1847,6 +1857,7 @@ unsigned long long gd_kernel_launches(void)
 
 int64_t gd_sort_kmers(gd_context* c, int slot)
 {
+    Turn turn(c->turn);
     if (slot < 0 || slot > 2 || !c->slot[slot].loaded)
     {
         gd_set_error("slot %d not loaded", slot);
@@ -1872,6 +1883,7 @@ int64_t gd_sort_kmers(gd_context* c, int slot)
 
 int64_t gd_get_kmers(gd_context* c, int slot, uint64_t* code, int32_t* read, int32_t* rpos, int64_t cap)
 {
+    Turn turn(c->turn);
     Slot& s = c->slot[slot];
     if (s.nk < 0)
     {
@@ -1895,6 +1907,7 @@ int64_t gd_get_kmers(gd_context* c, int slot, uint64_t* code, int32_t* read, int
 
 int gd_match_filter(gd_context* c, int bslot, int comp, int self)
 {
+    Turn turn(c->turn);
     if (c->variant != 1)
     {
         gd_set_error("gd_match_filter runs daligner's filter; daligner2 mode uses gd_match_filter2");
@@ -1948,6 +1961,7 @@ int gd_set_variant(gd_context* c, int variant, int hgap)
 
 int gd_match_filter2(gd_context* c, int bslot, int cslot, int self)
 {
+    Turn turn(c->turn);
     if (c->variant != 2)
     {
         gd_set_error("gd_match_filter2 needs gd_set_variant(ctx, 2, ...)");
@@ -2041,6 +2055,7 @@ int gd_test_handle_redundancies_d2(gd_context* c, const uint8_t* aseq, const uin
 
 int64_t gd_get_hits(gd_context* c, int32_t* rows4, int64_t cap)
 {
+    Turn turn(c->turn);
     int64_t n = std::min(c->nhits, cap);
     if (n <= 0)
         return c->nhits;
@@ -2060,6 +2075,7 @@ int64_t gd_get_hits(gd_context* c, int32_t* rows4, int64_t cap)
 
 int64_t gd_num_overlaps(gd_context* c, int64_t* trace_bytes)
 {
+    Turn turn(c->turn);
     if (trace_bytes)
         *trace_bytes = (int64_t)c->acc_tb;
     return (int64_t)c->acc_n;
@@ -2067,6 +2083,7 @@ int64_t gd_num_overlaps(gd_context* c, int64_t* trace_bytes)
 
 int64_t gd_sort_overlaps(gd_context* c, int64_t* trace_bytes)
 {
+    Turn turn(c->turn);
     if (sort_overlaps(c))
         return -1;
     if (trace_bytes)
@@ -2205,11 +2222,13 @@ static int64_t las_sort_files(gd_context* c, const char* const* in_paths, int ni
 
 int64_t gd_las_sort(gd_context* c, const char* in_path, const char* out_path)
 {
+    Turn turn(c->turn);
     return las_sort_files(c, &in_path, 1, out_path, 0);
 }
 
 int64_t gd_las_merge(gd_context* c, const char* const* in_paths, int nin, const char* out_path)
 {
+    Turn turn(c->turn);
     if (nin <= 0)
     {
         gd_set_error("gd_las_merge: no input files");
@@ -2222,6 +2241,7 @@ int64_t gd_dust(gd_context* c, int slot, int window, double thresh, int mflag, i
                 int64_t* anno, int32_t* data, int64_t cap)
 {
     using namespace gd;
+    Turn turn(c->turn);
     if (slot < 0 || slot > 2 || !c->slot[slot].loaded)
     {
         gd_set_error("gd_dust: slot %d not loaded", slot);
@@ -2297,6 +2317,7 @@ int64_t gd_dust(gd_context* c, int slot, int window, double thresh, int mflag, i
 
 int64_t gd_get_overlaps(gd_context* c, gd_overlap* recs, uint8_t* trace, int64_t rcap, int64_t tcap)
 {
+    Turn turn(c->turn);
     if (sort_overlaps(c))
         return -1;
     int64_t m = std::min<int64_t>(rcap, (int64_t)c->srt_n);
@@ -2334,6 +2355,7 @@ int64_t gd_get_overlaps(gd_context* c, gd_overlap* recs, uint8_t* trace, int64_t
 
 int gd_write_overlap_buffer(gd_context* c, int run_id, const char* ablock, const char* bblock, int last_read)
 {
+    Turn turn(c->turn);
     if (stage_sorted(c))
         return -1;
     const size_t nsrt = c->srt_n;
@@ -2435,6 +2457,7 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
                          int64_t n, int32_t* diffs_out)
 {
     using namespace gd;
+    Turn turn(c->turn);
     if (aslot < 0 || aslot > 2 || bslot < 0 || bslot > 2 || cslot < 0 || cslot > 2 || !c->slot[aslot].loaded ||
         !c->slot[bslot].loaded)
     {
@@ -2539,6 +2562,7 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
 
 int gd_reset_overlap_buffer(gd_context* c)
 {
+    Turn turn(c->turn);
     c->acc_n = c->acc_tb = 0;
     c->srt_n = c->srt_tb = 0;
     c->srt_valid = false;
@@ -2621,6 +2645,7 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
                              int32_t* out12, uint16_t* trace, int trstride, int64_t* cells)
 {
     using namespace gd;
+    Turn turn(c->turn);
     if (!c->spec_set)
     {
         gd_set_error("gd_new_align_spec has not been called");
@@ -2765,6 +2790,7 @@ int gd_triage_reset(gd_context* c)
 
 int gd_triage_set_model(gd_context* c, const float* params, float threshold)
 {
+    Turn turn(c->turn);
     if (!params)
     {
         c->tri_on = 0;
@@ -2787,6 +2813,7 @@ int gd_triage_set_model(gd_context* c, const float* params, float threshold)
 
 int gd_mlp_forward(gd_context* c, const float* params, const float* feat, int64_t n, float* prob)
 {
+    Turn turn(c->turn);
     if (n < 0)
     {
         gd_set_error("gd_mlp_forward: negative row count");
@@ -2809,6 +2836,7 @@ int gd_mlp_forward(gd_context* c, const float* params, const float* feat, int64_
 int gd_mlp_grad(gd_context* c, const float* params, const float* feat, const float* label, int n, float pos_weight,
                 float* grad, float* loss)
 {
+    Turn turn(c->turn);
     if (n <= 0)
     {
         gd_set_error("gd_mlp_grad: empty batch");
@@ -2879,6 +2907,7 @@ int gd_mlp_train(gd_context* c, const float* feat, const float* label, int64_t n
                  float pos_weight, uint64_t seed, float* params, float* epoch_loss)
 {
     using namespace gd;
+    Turn turn(c->turn);
     if (n <= 0 || batch <= 0 || epochs <= 0 || n > INT32_MAX)
     {
         gd_set_error("gd_mlp_train: bad sizes (n %lld, batch %d, epochs %d)", (long long)n, batch, epochs);
