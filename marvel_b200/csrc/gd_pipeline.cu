@@ -2471,8 +2471,12 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
     Slot& Cc = c->slot[cslot];
     const int TS = c->tspace;
     const int tbytes = TS <= 125 ? 1 : 2;
-    // the records' checks, their segments' places and the extent of their trace bytes
-    bool any_comp = false;
+    // the records' checks, their segments' places and the extent of their trace bytes: one piece of
+    // memory as long as every record's bytes lie within TRACE_GAP of those before it (a buffer as
+    // gd_get_overlaps fills it, from any record on); what lies between others is not read
+    constexpr uint64_t TRACE_GAP = 64;
+    bool any_comp = false, apart = false;
+    uint64_t used = 0;
     std::vector<int64_t> first(n + 1);
     int64_t nseg = 0;
     uint64_t tlo = UINT64_MAX, thi = 0;
@@ -2497,8 +2501,11 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
         nseg += inner + 1;
         if (inner)
         {
+            const uint64_t end = o.toff + (uint64_t)2 * inner * tbytes;
+            apart = apart || (thi > tlo && (o.toff > thi + TRACE_GAP || end + TRACE_GAP < tlo));
             tlo = std::min(tlo, o.toff);
-            thi = std::max(thi, o.toff + (uint64_t)2 * inner * tbytes);
+            thi = std::max(thi, end);
+            used += end - o.toff;
         }
     }
     first[n] = nseg;
@@ -2509,6 +2516,26 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
     }
     if (thi <= tlo)
         tlo = thi = 0;
+    std::vector<gd_overlap> own;  // records apart: their bytes one after the other, and copies that say where
+    std::vector<uint8_t> bytes;
+    if (apart)
+    {
+        own.assign(recs, recs + n);
+        bytes.resize(used);
+        used = 0;
+        for (gd_overlap& o : own)
+        {
+            const uint64_t len = (uint64_t)2 * trace_inner(o.tlen) * tbytes;
+            if (len)
+                memcpy(bytes.data() + used, trace + o.toff, len);
+            o.toff = used;
+            used += len;
+        }
+        recs = own.data();
+        trace = bytes.data();
+        tlo = 0;
+        thi = used;
+    }
     const DevBlock& Cb = Cc.loaded ? Cc.blk : B.blk;
     cudaStream_t s = c->s;
     const int plain = slots_plain(c, {&A, &B, &Cc});
