@@ -45,10 +45,19 @@ void gd_set_error(const char* fmt, ...)
 namespace
 {
 
+// device memory, freed with its owner
 struct DevBuf
 {
     void* p = nullptr;
     size_t n = 0;
+    DevBuf() = default;
+    DevBuf(const DevBuf&) = delete;
+    DevBuf& operator=(const DevBuf&) = delete;
+    ~DevBuf()
+    {
+        if (p)
+            cudaFree(p);
+    }
 };
 
 int ensure(DevBuf& b, size_t bytes)
@@ -71,14 +80,6 @@ int ensure(DevBuf& b, size_t bytes)
     }
     b.n = want;
     return 0;
-}
-
-void release(DevBuf& b)
-{
-    if (b.p)
-        cudaFree(b.p);
-    b.p = nullptr;
-    b.n = 0;
 }
 
 template <typename T>
@@ -1597,30 +1598,10 @@ void gd_destroy(gd_context* c)
     if (!c)
         return;
     cudaStreamSynchronize(c->s);
-    DevBuf* bufs[] = {&c->tables, &c->k0,     &c->v0,    &c->k1,     &c->v1,     &c->scratch, &c->flags,
-                      &c->excl,   &c->jb,     &c->cnt,   &c->hoff,   &c->ctrun,  &c->gram,    &c->misc,
-                      &c->hk0,    &c->hd0,    &c->hk1,   &c->hd1,    &c->starts, &c->groups,  &c->gcost,
-                      &c->gidx,   &c->gcost2, &c->gidx2, &c->ascr,   &c->outrec, &c->outtr,   &c->counters,
-                      &c->status, &c->queue,  &c->tri_params, &c->tri_feat, &c->tri_prob, &c->tri_skip,
-                      &c->tri_gstat, &c->tri_misc, &c->tri_x, &c->tri_y, &c->tri_perm, &c->tri_grad, &c->tri_m,
-                      &c->tri_v, &c->tri_loss, &c->tri_w, &c->acc_rec, &c->acc_tr, &c->srt_rec, &c->srt_tr,
-                      &c->okey0, &c->okey1, &c->oval0, &c->oval1, &c->olen, &c->las_raw, &c->las_off,
-                      &c->las_rec, &c->las_out, &c->ascr_w, &c->wide, &c->ascr_d, &c->vf_rec, &c->vf_first,
-                      &c->vf_trace, &c->vf_seg, &c->vf_list, &c->vf_diff, &c->vf_misc, &c->vf_scr, &c->lb_a, &c->lb_b,
-                      &c->lb_pka, &c->lb_pkb, &c->lb_in, &c->lb_out, &c->lb_tr,
-                      &c->ah_path, &c->ah_misc, &c->ah_trace};
-    for (DevBuf* b : bufs)
-        release(*b);
     for (HostBuf* h : {&c->h_rec, &c->h_tr})
         if (h->p)
             cudaFreeHost(h->p);
     release(c->stage);
-    for (Slot& s : c->slot)
-    {
-        DevBuf* sb[] = {&s.bases, &s.boff, &s.rlen, &s.manno, &s.mdata, &s.code, &s.read, &s.rpos};
-        for (DevBuf* b : sb)
-            release(*b);
-    }
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
     cudaEventDestroy(c->tev0);
@@ -2001,16 +1982,6 @@ int gd_test_handle_redundancies_d2(gd_context* c, const uint8_t* aseq, const uin
     const int pcap_tr = (int)(ttot + 8 * (int64_t)(m / tspace + 8) * npath + 4096);
     const int vcap = 4 * m + 64, btcap = 2 * (m / tspace + 8) + 64;
     DevBuf da, db, dh, dp, dt, dv, dbt, doh, dn;
-    struct Frees  // the hook's buffers are its own; cudaFree waits for the device
-    {
-        DevBuf* b[9];
-        ~Frees()
-        {
-            for (DevBuf* x : b)
-                if (x->p)
-                    cudaFree(x->p);
-        }
-    } frees{{&da, &db, &dh, &dp, &dt, &dv, &dbt, &doh, &dn}};
     if (ensure(da, alen + 2) || ensure(db, blen + 2) || ensure(dh, npath * 24) ||
         ensure(dp, (npath + 1) * sizeof(MPath)) || ensure(dt, (size_t)pcap_tr * 2) || ensure(dv, (size_t)vcap * 4) ||
         ensure(dbt, (size_t)btcap * 2) || ensure(doh, (size_t)npath * 7 * 4) || ensure(dn, 4))
