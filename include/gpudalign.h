@@ -191,6 +191,10 @@ int gd_set_capacities(gd_context* ctx, int pebbles, int traces, int paths, int64
  * sort makes afterwards must report it (-1, gd_last_error set) and clear it. */
 int gd_test_wait_expiry(gd_context* ctx, int polls);
 
+/* Test hook: from now on an allocation that would take the context's device buffers beyond bytes
+ * fails, as cudaMalloc does when memory runs out (0: no limit).  Returns the bytes they hold now. */
+int64_t gd_test_memory_limit(gd_context* ctx, int64_t bytes);
+
 /* LAsort (dalign/LAsort.c:65-90, 139-256) of one .las file on the device: writes out_path
  * with the records of in_path ordered by (aread, bread, abpos) -- ties, which the
  * reference's qsort leaves unordered, by (aepos, bbpos) and then file order -- each record's

@@ -63,7 +63,8 @@ SYMBOLS = ["gd_create", "gd_destroy", "gd_last_error", "gd_set_filter_params", "
            "gd_compute_trace_pts", "gd_triage_collect", "gd_triage_get_groups", "gd_triage_reset",
            "gd_triage_set_model", "gd_mlp_init", "gd_mlp_forward", "gd_mlp_grad", "gd_mlp_train", "gd_sort_overlaps", "gd_las_sort", "gd_dust", "gd_las_merge",
            "gd_set_wave_limit", "gd_set_variant", "gd_match_filter2", "gd_test_handle_redundancies_d2",
-           "gd_set_biased", "gd_set_capacities", "gd_test_wait_expiry", "gd_set_align_schedule"]
+           "gd_set_biased", "gd_set_capacities", "gd_test_wait_expiry", "gd_set_align_schedule",
+           "gd_test_memory_limit"]
 
 TRI_NF = 12        # features per pair group
 TRI_NPARAM = 5081  # model parameter vector (gd_triage_set_model)
@@ -107,6 +108,8 @@ def lib():
     L.gd_set_wave_limit.argtypes = [C.c_void_p, C.c_int]
     L.gd_set_capacities.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int64, C.c_int64]
     L.gd_test_wait_expiry.argtypes = [C.c_void_p, C.c_int]
+    L.gd_test_memory_limit.argtypes = [C.c_void_p, C.c_int64]
+    L.gd_test_memory_limit.restype = C.c_int64
     L.gd_set_align_schedule.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
     L.gd_dust.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_double, C.c_int, C.c_int, C.POINTER(C.c_float),
                           C.c_void_p, C.c_void_p, C.c_int64]
@@ -365,6 +368,11 @@ class Context:
         returns (status of the sort's wait check, its error text)."""
         rc = lib().gd_test_wait_expiry(self.h, int(polls))
         return rc, (lib().gd_last_error() or b"").decode()
+
+    def test_memory_limit(self, limit=0):
+        """Test hook: the context's device buffers may hold this many bytes (0: no limit); returns
+        what they hold now."""
+        return _check(lib().gd_test_memory_limit(self.h, int(limit)))
 
     def las_merge(self, in_paths, out_path):
         """LAmerge of .las files on the device; returns the number of records."""

@@ -60,24 +60,21 @@ struct DevBuf
     }
 };
 
+// cudaMalloc for the context whose call runs in this thread: what the context keeps without
+// need is freed when memory runs out
+int dev_malloc(void** p, size_t bytes);
+void dev_free(DevBuf& b);
+
 int ensure(DevBuf& b, size_t bytes)
 {
     if (bytes == 0)
         bytes = 16;
     if (bytes <= b.n)
         return 0;
-    if (b.p)
-        cudaFree(b.p);
-    b.p = nullptr;
-    b.n = 0;
-    size_t want = bytes + bytes / 8;
-    cudaError_t e = cudaMalloc(&b.p, want);
-    if (e != cudaSuccess)
-    {
-        b.p = nullptr;
-        gd_set_error("cudaMalloc of %zu bytes failed: %s", want, cudaGetErrorString(e));
+    dev_free(b);
+    const size_t want = bytes + bytes / 8;
+    if (dev_malloc(&b.p, want))
         return -1;
-    }
     b.n = want;
     return 0;
 }
@@ -95,19 +92,14 @@ int ensure_keep(DevBuf& b, size_t bytes, size_t used, cudaStream_t s)
         return 0;
     size_t want = bytes + bytes / 2;
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, want);
-    if (e != cudaSuccess)
-    {
-        gd_set_error("cudaMalloc of %zu bytes failed: %s", want, cudaGetErrorString(e));
+    if (dev_malloc(&p, want))
         return -1;
-    }
     if (used)
     {
         GD_CUDA(cudaMemcpyAsync(p, b.p, used, cudaMemcpyDeviceToDevice, s));
         GD_CUDA(cudaStreamSynchronize(s));
     }
-    if (b.p)
-        cudaFree(b.p);
+    dev_free(b);
     b.p = p;
     b.n = want;
     return 0;
@@ -334,6 +326,18 @@ struct gd_context
     DevBuf las_raw, las_off, las_rec, las_out;  // gd_las_sort
     DevBuf lb_a, lb_b, lb_pka, lb_pkb, lb_in, lb_out, lb_tr;  // gd_local_alignment_batch
     DevBuf vf_rec, vf_first, vf_trace, vf_seg, vf_list, vf_diff, vf_misc, vf_scr;  // gd_compute_trace_pts
+    // buffers that hold nothing between calls: freed when memory runs out while no call uses them
+    struct Kept
+    {
+        std::vector<DevBuf*> bufs;
+        bool busy = false;
+    };
+    Kept kept_lb{{&lb_a, &lb_b, &lb_pka, &lb_pkb, &lb_in, &lb_out, &lb_tr}};
+    Kept kept_vf{{&vf_rec, &vf_first, &vf_trace, &vf_seg, &vf_list, &vf_diff, &vf_misc, &vf_scr}};
+    Kept kept_ah{{&ah_path, &ah_misc, &ah_trace}};
+    Kept kept_scr{{&ascr, &ascr_w, &ascr_d}};
+    size_t held = 0;   // bytes of this context's buffers
+    size_t limit = 0;  // tests only: beyond this many bytes an allocation fails
     gd_stats stats;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, tev0 = nullptr, tev1 = nullptr;
     // learned triage: model (on), per-group feature/outcome collection (collect)
@@ -345,7 +349,99 @@ struct gd_context
     std::vector<uint32_t> tri_hrec, tri_hcells;
 };
 
-using Turn = std::lock_guard<std::recursive_mutex>;
+// A call's turn on its context
+struct Turn
+{
+    std::lock_guard<std::recursive_mutex> lock;
+    gd_context* const before;
+    static thread_local gd_context* now;  // the context whose call runs in this thread
+    explicit Turn(gd_context* c) : lock(c->turn), before(now)
+    {
+        now = c;
+    }
+    ~Turn()
+    {
+        now = before;
+    }
+};
+thread_local gd_context* Turn::now = nullptr;
+
+// A call's use of kept buffers.  On return those that together exceed most bytes are freed (0: none are):
+// a call frees what it does not leave to the next one of its kind, as all of it was before
+// buffers were kept.
+struct InUse
+{
+    gd_context::Kept& k;
+    const size_t most;
+    InUse(gd_context::Kept& kept, size_t keep) : k(kept), most(keep)
+    {
+        k.busy = true;
+    }
+    ~InUse();
+};
+
+// what a batch or a trace check leaves at most: the buffers of 4,000 seeds (150 MB) or of 45,000
+// records (100 MB), whose allocation cost as much as the call
+constexpr size_t KEPT_BYTES = 256u << 20;
+
+namespace
+{
+
+void dev_free(DevBuf& b)
+{
+    if (!b.p)
+        return;
+    cudaFree(b.p);
+    if (Turn::now)
+        Turn::now->held -= b.n;
+    b.p = nullptr;
+    b.n = 0;
+}
+
+int dev_malloc(void** p, size_t bytes)
+{
+    gd_context* const c = Turn::now;
+    auto attempt = [&]() {
+        *p = nullptr;
+        if (c && c->limit && c->held + bytes > c->limit)
+            return cudaErrorMemoryAllocation;
+        const cudaError_t e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess)
+            cudaGetLastError();  // reported here, not by the next launch's check
+        return e;
+    };
+    cudaError_t e = attempt();
+    if (e == cudaErrorMemoryAllocation && c)
+    {
+        for (gd_context::Kept* k : {&c->kept_lb, &c->kept_vf, &c->kept_ah, &c->kept_scr})
+            if (!k->busy)
+                for (DevBuf* b : k->bufs)
+                    dev_free(*b);
+        e = attempt();
+    }
+    if (e != cudaSuccess)
+    {
+        *p = nullptr;
+        gd_set_error("cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+        return -1;
+    }
+    if (c)
+        c->held += bytes;
+    return 0;
+}
+
+}  // namespace
+
+InUse::~InUse()
+{
+    k.busy = false;
+    size_t n = 0;
+    for (DevBuf* b : k.bufs)
+        n += b->n;
+    if (most && n > most)
+        for (DevBuf* b : k.bufs)
+            dev_free(*b);
+}
 
 // ----------------------------------------------------------------------------------------
 // align spec: trim tables (set_table / New_Align_Spec, dalign/align.c:196-279)
@@ -1027,6 +1123,7 @@ constexpr size_t AHEAD_TRACE = 48u << 20;
 static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBits hb, int comp, int self)
 {
     using namespace gd;
+    InUse scratch_use(c->kept_scr, 0), ahead_use(c->kept_ah, 0);
     cudaStream_t s = c->s;
     const int oi = comp ? 1 : 0;
     const int hbits = hb.pbits + hb.abits + hb.bbits;
@@ -1634,7 +1731,7 @@ int gd_set_filter_params(gd_context* c, int kmer, int binshift, int suppress, in
 int gd_new_align_spec(gd_context* c, double ave_corr, int trace_space, const float freq[4], int symmetric,
                       int only_identity, int no_trace_points)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (trace_space <= 0)
     {
         gd_set_error("invalid trace spacing of (%d)", trace_space);
@@ -1664,7 +1761,7 @@ static int pack_slot(gd_context* c, Slot& s, int64_t nbytes);
 
 int gd_load_block(gd_context* c, int slot, const gd_block* b)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (slot < 0 || slot > 2)
     {
         gd_set_error("slot %d out of range", slot);
@@ -1763,7 +1860,7 @@ static int pack_slot(gd_context* c, Slot& s, int64_t nbytes)
 
 int gd_complement_block(gd_context* c, int src, int dst)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (src < 0 || src > 2 || dst < 0 || dst > 2 || src == dst || !c->slot[src].loaded)
     {
         gd_set_error("bad complement slots %d -> %d", src, dst);
@@ -1838,7 +1935,7 @@ unsigned long long gd_kernel_launches(void)
 
 int64_t gd_sort_kmers(gd_context* c, int slot)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (slot < 0 || slot > 2 || !c->slot[slot].loaded)
     {
         gd_set_error("slot %d not loaded", slot);
@@ -1864,7 +1961,7 @@ int64_t gd_sort_kmers(gd_context* c, int slot)
 
 int64_t gd_get_kmers(gd_context* c, int slot, uint64_t* code, int32_t* read, int32_t* rpos, int64_t cap)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     Slot& s = c->slot[slot];
     if (s.nk < 0)
     {
@@ -1888,7 +1985,7 @@ int64_t gd_get_kmers(gd_context* c, int slot, uint64_t* code, int32_t* read, int
 
 int gd_match_filter(gd_context* c, int bslot, int comp, int self)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (c->variant != 1)
     {
         gd_set_error("gd_match_filter runs daligner's filter; daligner2 mode uses gd_match_filter2");
@@ -1942,7 +2039,7 @@ int gd_set_variant(gd_context* c, int variant, int hgap)
 
 int gd_match_filter2(gd_context* c, int bslot, int cslot, int self)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (c->variant != 2)
     {
         gd_set_error("gd_match_filter2 needs gd_set_variant(ctx, 2, ...)");
@@ -2026,7 +2123,7 @@ int gd_test_handle_redundancies_d2(gd_context* c, const uint8_t* aseq, const uin
 
 int64_t gd_get_hits(gd_context* c, int32_t* rows4, int64_t cap)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     int64_t n = std::min(c->nhits, cap);
     if (n <= 0)
         return c->nhits;
@@ -2046,7 +2143,7 @@ int64_t gd_get_hits(gd_context* c, int32_t* rows4, int64_t cap)
 
 int64_t gd_num_overlaps(gd_context* c, int64_t* trace_bytes)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (trace_bytes)
         *trace_bytes = (int64_t)c->acc_tb;
     return (int64_t)c->acc_n;
@@ -2054,7 +2151,7 @@ int64_t gd_num_overlaps(gd_context* c, int64_t* trace_bytes)
 
 int64_t gd_sort_overlaps(gd_context* c, int64_t* trace_bytes)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (sort_overlaps(c))
         return -1;
     if (trace_bytes)
@@ -2193,13 +2290,13 @@ static int64_t las_sort_files(gd_context* c, const char* const* in_paths, int ni
 
 int64_t gd_las_sort(gd_context* c, const char* in_path, const char* out_path)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     return las_sort_files(c, &in_path, 1, out_path, 0);
 }
 
 int64_t gd_las_merge(gd_context* c, const char* const* in_paths, int nin, const char* out_path)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (nin <= 0)
     {
         gd_set_error("gd_las_merge: no input files");
@@ -2212,7 +2309,7 @@ int64_t gd_dust(gd_context* c, int slot, int window, double thresh, int mflag, i
                 int64_t* anno, int32_t* data, int64_t cap)
 {
     using namespace gd;
-    Turn turn(c->turn);
+    Turn turn(c);
     if (slot < 0 || slot > 2 || !c->slot[slot].loaded)
     {
         gd_set_error("gd_dust: slot %d not loaded", slot);
@@ -2288,7 +2385,7 @@ int64_t gd_dust(gd_context* c, int slot, int window, double thresh, int mflag, i
 
 int64_t gd_get_overlaps(gd_context* c, gd_overlap* recs, uint8_t* trace, int64_t rcap, int64_t tcap)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (sort_overlaps(c))
         return -1;
     int64_t m = std::min<int64_t>(rcap, (int64_t)c->srt_n);
@@ -2326,7 +2423,7 @@ int64_t gd_get_overlaps(gd_context* c, gd_overlap* recs, uint8_t* trace, int64_t
 
 int gd_write_overlap_buffer(gd_context* c, int run_id, const char* ablock, const char* bblock, int last_read)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (stage_sorted(c))
         return -1;
     const size_t nsrt = c->srt_n;
@@ -2428,7 +2525,7 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
                          int64_t n, int32_t* diffs_out)
 {
     using namespace gd;
-    Turn turn(c->turn);
+    Turn turn(c);
     if (aslot < 0 || aslot > 2 || bslot < 0 || bslot > 2 || cslot < 0 || cslot > 2 || !c->slot[aslot].loaded ||
         !c->slot[bslot].loaded)
     {
@@ -2509,6 +2606,7 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
     }
     const DevBlock& Cb = Cc.loaded ? Cc.blk : B.blk;
     cudaStream_t s = c->s;
+    InUse use(c->kept_vf, KEPT_BYTES);
     const int plain = slots_plain(c, {&A, &B, &Cc});
     if (plain < 0)
         return -1;
@@ -2560,7 +2658,7 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
 
 int gd_reset_overlap_buffer(gd_context* c)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     c->acc_n = c->acc_tb = 0;
     c->srt_n = c->srt_tb = 0;
     c->srt_valid = false;
@@ -2625,6 +2723,13 @@ int gd_test_wait_expiry(gd_context* c, int polls)
     return gd::radix_sort_wait_check(c->s);
 }
 
+int64_t gd_test_memory_limit(gd_context* c, int64_t bytes)
+{
+    Turn turn(c);
+    c->limit = (size_t)std::max<int64_t>(0, bytes);
+    return (int64_t)c->held;
+}
+
 int gd_get_stats(gd_context* c, gd_stats* st)
 {
     c->stats.records = (int64_t)c->acc_n;
@@ -2643,7 +2748,7 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
                              int32_t* out12, uint16_t* trace, int trstride, int64_t* cells)
 {
     using namespace gd;
-    Turn turn(c->turn);
+    Turn turn(c);
     if (!c->spec_set)
     {
         gd_set_error("gd_new_align_spec has not been called");
@@ -2690,6 +2795,7 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     AlignScratch sc{};
     // the context keeps these buffers (the scratch is the pair aligner's); the call's own cudaMalloc
     // and cudaFree of 2 GB took most of its time
+    InUse use(c->kept_lb, KEPT_BYTES), scratch_use(c->kept_scr, 0);
     const size_t n8 = (size_t)nseeds * 8, n4 = (size_t)nseeds * 4;
     const int64_t wa = (abytes + 15) / 16 + 1, wb = (bbytes + 15) / 16 + 1;
     if (ensure(c->lb_a, abytes) || ensure(c->lb_b, bbytes) || ensure(c->lb_pka, wa * 4) ||
@@ -2788,7 +2894,7 @@ int gd_triage_reset(gd_context* c)
 
 int gd_triage_set_model(gd_context* c, const float* params, float threshold)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (!params)
     {
         c->tri_on = 0;
@@ -2811,7 +2917,7 @@ int gd_triage_set_model(gd_context* c, const float* params, float threshold)
 
 int gd_mlp_forward(gd_context* c, const float* params, const float* feat, int64_t n, float* prob)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (n < 0)
     {
         gd_set_error("gd_mlp_forward: negative row count");
@@ -2834,7 +2940,7 @@ int gd_mlp_forward(gd_context* c, const float* params, const float* feat, int64_
 int gd_mlp_grad(gd_context* c, const float* params, const float* feat, const float* label, int n, float pos_weight,
                 float* grad, float* loss)
 {
-    Turn turn(c->turn);
+    Turn turn(c);
     if (n <= 0)
     {
         gd_set_error("gd_mlp_grad: empty batch");
@@ -2905,7 +3011,7 @@ int gd_mlp_train(gd_context* c, const float* feat, const float* label, int64_t n
                  float pos_weight, uint64_t seed, float* params, float* epoch_loss)
 {
     using namespace gd;
-    Turn turn(c->turn);
+    Turn turn(c);
     if (n <= 0 || batch <= 0 || epochs <= 0 || n > INT32_MAX)
     {
         gd_set_error("gd_mlp_train: bad sizes (n %lld, batch %d, epochs %d)", (long long)n, batch, epochs);

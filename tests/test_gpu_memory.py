@@ -1,4 +1,4 @@
-"""Device memory of a context: all of it returns when it is destroyed."""
+"""Device memory of a context: what its calls keep, and that all of it returns when it is destroyed."""
 import numpy as np
 import pytest
 
@@ -46,3 +46,81 @@ def test_destroy_frees_everything():
     for _ in range(3):
         cycle()
     assert before - free() < 4 << 20
+
+
+def one_read(n):
+    bases = np.full(n + 2, 4, np.uint8)
+    bases[1:-1] = np.random.default_rng(n).integers(0, 4, n, dtype=np.uint8)
+    return dazzdb.Block(bases, np.array([0, n + 1], np.int64), np.array([n], np.int32), 0, 1, np.full(4, .25, np.float32),
+                        n, n)
+
+
+def big_check(ctx, nrec, blk, ts=2):
+    """nrec records of the read against itself, all with the same trace"""
+    import marvel_b200 as mb
+    n = int(blk.rlen[0])
+    r = np.zeros(nrec, mb.OVL_DTYPE)
+    r["aepos"] = r["bepos"] = n
+    r["tlen"] = 2 * (n // ts)
+    tr = np.tile(np.array([0, ts], np.uint8), n // ts)
+    assert not ctx.compute_trace_pts(r, tr, 0, 0, 0).any()
+
+
+def big_batch(ctx, nseeds, stride, blk):
+    z = np.zeros(nseeds, np.int32)
+    n = np.full(nseeds, blk.rlen[0], np.int32)
+    out, _, _ = ctx.local_alignment_batch(blk.bases, z + 1, n, blk.bases.copy(), z + 1, n, z, z, 0, stride)
+    assert (out[:, 2] == n[0]).all()
+
+
+def test_large_calls_return_their_memory():
+    """A trace check of 20 M segments (36 bytes each) and a batch with 1 GB of trace rows keep
+    less than 300 MB beyond what a small one keeps."""
+    import marvel_b200 as mb
+    ctx = mb.Context()
+    ctx.set_filter_params()
+    blk = one_read(20000)
+    ctx.new_align_spec(0.70, 2, blk.freq)
+    ctx.load_block(0, blk)
+    big_check(ctx, 2, blk)
+    before = free()
+    big_check(ctx, 2000, blk)
+    assert before - free() < 300 << 20
+    ctx.new_align_spec(0.70, 100, blk.freq)
+    big_batch(ctx, 500, 2000, blk)
+    before = free()
+    big_batch(ctx, 500, 1 << 20, blk)
+    assert before - free() < 300 << 20
+    ctx.close()
+
+
+def test_kept_memory_is_freed_for_a_call_that_needs_it():
+    """Buffers that a seed batch and a trace check left do not stand in the way of a block, an index or a
+    comparison."""
+    import marvel_b200 as mb
+    small, blk = one_read(20000), random_block(np.random.default_rng(1), 1500, 6000)
+    plain = mb.Context()
+    want = mb.daligner_block(plain, blk)
+    need = plain.test_memory_limit()
+    plain.close()
+    ctx = mb.Context()
+    ctx.set_filter_params()
+    ctx.new_align_spec(0.70, 2, small.freq)
+    ctx.load_block(0, small)
+    big_check(ctx, 300, small)
+    ctx.new_align_spec(0.70, 100, small.freq)
+    big_batch(ctx, 500, 100000, small)
+    kept = ctx.test_memory_limit()
+    assert kept > 200 << 20
+    ctx.test_memory_limit(need + (8 << 20))
+    got = mb.daligner_block(ctx, blk)
+    assert got[0].tobytes() == want[0].tobytes() and got[1].tobytes() == want[1].tobytes()
+    held = ctx.test_memory_limit(need // 2)  # what does not fit either way is an error, and the context goes on
+    assert held <= need + (8 << 20)
+    with pytest.raises(mb.GpuError, match="cudaMalloc"):
+        big_batch(ctx, 500, 4 << 20, small)
+    ctx.test_memory_limit(0)
+    big_batch(ctx, 20, 2000, small)
+    got = mb.daligner_block(ctx, blk)
+    assert got[0].tobytes() == want[0].tobytes() and got[1].tobytes() == want[1].tobytes()
+    ctx.close()
