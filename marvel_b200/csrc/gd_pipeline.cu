@@ -1357,14 +1357,19 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
                      c->tbcap, skip, c->tri_collect ? P<uint2>(c->tri_gstat) : nullptr, wide_list, d_nwide,
                      Ahead{}};
         GD_CUDA(cudaEventRecord(c->ev0, s));
-        if (nheavy)
+        // without room for them no seeds are aligned ahead: the plain pair kernel aligns all
+        c->kept_ah.busy = true;
+        const bool ahead = nheavy && !ensure(c->ah_path, AHEAD_CAP * sizeof(AheadPath)) &&
+                           !ensure(c->ah_trace, AHEAD_TRACE * 2) &&
+                           !ensure(c->ah_misc, AHEAD_GROUPS * sizeof(uint2) + 16 + sizeof(DevStatus));
+        if (nheavy && !ahead)
+            for (DevBuf* b : c->kept_ah.bufs)
+                dev_free(*b);
+        if (ahead)
         {
             bool any = false;
             Ahead ah{};
             ah.cap = AHEAD_TRACE;
-            if (ensure(c->ah_path, AHEAD_CAP * sizeof(AheadPath)) || ensure(c->ah_trace, AHEAD_TRACE * 2) ||
-                ensure(c->ah_misc, AHEAD_GROUPS * sizeof(uint2) + 16 + sizeof(DevStatus)))
-                return -1;
             ah.path = P<AheadPath>(c->ah_path);
             ah.trace = P<uint16_t>(c->ah_trace);
             ah.groups = P<uint2>(c->ah_misc);
@@ -1395,6 +1400,7 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
         unsigned nwide = 0;
         GD_CUDA(cudaMemcpyAsync(&nwide, d_nwide, 4, cudaMemcpyDeviceToHost, s));
         GD_CUDA(cudaStreamSynchronize(s));
+        c->kept_ah.busy = false;  // the seeds are taken: what follows may have the memory
         c->stats.wide[oi] = nwide;
         if (nwide > 0)
         {

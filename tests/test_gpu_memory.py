@@ -124,3 +124,23 @@ def test_kept_memory_is_freed_for_a_call_that_needs_it():
     got = mb.daligner_block(ctx, blk)
     assert got[0].tobytes() == want[0].tobytes() and got[1].tobytes() == want[1].tobytes()
     ctx.close()
+
+
+def test_comparison_without_room_for_seeds_ahead():
+    """A block of tandem repeats, whose seeds are aligned ahead where there is room: without it they are
+    not, and the comparison gives the same."""
+    import marvel_b200 as mb
+    from test_gpu_ahead import block, reads
+    blk = block(reads(np.random.default_rng(7), 60, 3000, 8, 0.12, False))
+    ctx = mb.Context()
+    want = mb.daligner_block(ctx, blk)
+    need = ctx.test_memory_limit()
+    ctx.close()
+    for short in (60 << 20, 125 << 20):  # less than all of the seeds' buffers (136 MB), all but the smallest
+        ctx = mb.Context()
+        ctx.test_memory_limit(need - short)
+        for _ in range(2):
+            got = mb.daligner_block(ctx, blk)
+            assert got[0].tobytes() == want[0].tobytes() and got[1].tobytes() == want[1].tobytes()
+        assert ctx.test_memory_limit() <= need - short
+        ctx.close()
