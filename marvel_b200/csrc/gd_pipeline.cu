@@ -15,8 +15,6 @@
 #include <initializer_list>
 #include <mutex>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/gpudalign.h"
@@ -26,6 +24,7 @@
 #include "gd_dust.cuh"
 #include "gd_output.cuh"
 #include "gd_prims.cuh"
+#include "gd_staging.cuh"
 #include "gd_verify.cuh"
 #include "gd_triage.cuh"
 
@@ -133,119 +132,9 @@ int ensure_host(HostBuf& b, size_t bytes)
     return 0;
 }
 
-// Copies between device memory and pageable host memory through pinned staging: the driver's own
-// pageable path moves one small piece at a time (105 MB of bases took about 25 ms, and results
-// into fresh pages as long again).  STAGE_THREADS host threads take STAGE_CHUNK pieces in turn, each
-// with two pinned buffers, so that one piece's host copy (and the page faults of a fresh result
-// array) runs beside another's transfer.  Small copies and pinned memory go straight.
-constexpr size_t STAGE_CHUNK = 2u << 20;
-constexpr size_t STAGE_MIN = 4u << 20;  // below this the threads cost what they save
-constexpr int STAGE_THREADS = 4;
-
-struct Staging
-{
-    char* buf = nullptr;  // 2 pieces per thread, pinned
-    cudaEvent_t ev[2 * STAGE_THREADS] = {};
-};
-
-void release(Staging& g)
-{
-    for (cudaEvent_t e : g.ev)
-        if (e)
-            cudaEventDestroy(e);
-    if (g.buf)
-        cudaFreeHost(g.buf);
-    g = Staging{};
-}
-
-bool is_pageable(const void* p)
-{
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess)
-    {
-        cudaGetLastError();
-        return true;
-    }
-    return a.type == cudaMemoryTypeUnregistered;
-}
-
-// dev <-> host (to_dev), n bytes on stream s.  To the device: the host memory may be reused on
-// return, as after a pageable cudaMemcpyAsync.  To the host: complete on return.
 int staged_copy(Staging& g, void* dev, void* host, size_t n, bool to_dev, cudaStream_t s)
 {
-    if (n < STAGE_MIN || !is_pageable(host))
-    {
-        GD_CUDA(cudaMemcpyAsync(to_dev ? dev : host, to_dev ? host : dev, n,
-                                to_dev ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, s));
-        if (!to_dev)
-            GD_CUDA(cudaStreamSynchronize(s));
-        return 0;
-    }
-    if (!g.buf)
-    {
-        for (cudaEvent_t& e : g.ev)
-            GD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        GD_CUDA(cudaMallocHost((void**)&g.buf, 2 * STAGE_THREADS * STAGE_CHUNK));
-    }
-    int dev_id = 0;
-    GD_CUDA(cudaGetDevice(&dev_id));
-    cudaError_t errs[STAGE_THREADS] = {};
-    auto work = [&](int t) {
-        cudaError_t& e = errs[t];
-        if ((e = cudaSetDevice(dev_id)) != cudaSuccess)
-            return;
-        struct
-        {
-            size_t at = 0, len = 0;  // the piece in flight in this buffer
-        } fly[2];
-        auto land = [&](int b) {
-            if (fly[b].len == 0 || e != cudaSuccess)
-                return;
-            e = cudaEventSynchronize(g.ev[2 * t + b]);
-            if (e == cudaSuccess && !to_dev)
-                memcpy((char*)host + fly[b].at, g.buf + (2 * t + b) * STAGE_CHUNK, fly[b].len);
-            fly[b].len = 0;
-        };
-        int b = 0;
-        for (size_t at = t * STAGE_CHUNK; at < n && e == cudaSuccess; at += STAGE_THREADS * STAGE_CHUNK, b ^= 1)
-        {
-            land(b);
-            if (e != cudaSuccess)
-                return;
-            char* const pin = g.buf + (2 * t + b) * STAGE_CHUNK;
-            const size_t len = std::min(STAGE_CHUNK, n - at);
-            if (to_dev)
-            {
-                memcpy(pin, (const char*)host + at, len);
-                e = cudaMemcpyAsync((char*)dev + at, pin, len, cudaMemcpyHostToDevice, s);
-            }
-            else
-                e = cudaMemcpyAsync(pin, (const char*)dev + at, len, cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess)
-                e = cudaEventRecord(g.ev[2 * t + b], s);
-            fly[b].at = at;
-            fly[b].len = len;
-        }
-        land(b);
-        land(b ^ 1);
-    };
-    std::vector<std::thread> th;
-    for (int t = 1; t < STAGE_THREADS; t++)
-    {
-        try
-        {
-            th.emplace_back(work, t);
-        }
-        catch (const std::system_error&)
-        {
-            work(t);  // no thread to be had: its share here
-        }
-    }
-    work(0);
-    for (std::thread& x : th)
-        x.join();
-    for (cudaError_t e : errs)
-        GD_CUDA(e);
+    GD_CUDA(stage_copy(g, dev, host, n, to_dev, s));
     return 0;
 }
 
