@@ -64,7 +64,7 @@ SYMBOLS = ["gd_create", "gd_destroy", "gd_last_error", "gd_set_filter_params", "
            "gd_triage_set_model", "gd_mlp_init", "gd_mlp_forward", "gd_mlp_grad", "gd_mlp_train", "gd_sort_overlaps", "gd_las_sort", "gd_dust", "gd_las_merge",
            "gd_set_wave_limit", "gd_set_variant", "gd_match_filter2", "gd_test_handle_redundancies_d2",
            "gd_set_biased", "gd_set_capacities", "gd_test_wait_expiry", "gd_set_align_schedule",
-           "gd_test_memory_limit"]
+           "gd_test_memory_limit", "gd_test_ahead"]
 
 TRI_NF = 12        # features per pair group
 TRI_NPARAM = 5081  # model parameter vector (gd_triage_set_model)
@@ -110,6 +110,7 @@ def lib():
     L.gd_test_wait_expiry.argtypes = [C.c_void_p, C.c_int]
     L.gd_test_memory_limit.argtypes = [C.c_void_p, C.c_int64]
     L.gd_test_memory_limit.restype = C.c_int64
+    L.gd_test_ahead.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p]
     L.gd_set_align_schedule.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
     L.gd_dust.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_double, C.c_int, C.c_int, C.POINTER(C.c_float),
                           C.c_void_p, C.c_void_p, C.c_int64]
@@ -373,6 +374,13 @@ class Context:
         """Test hook: the context's device buffers may hold this many bytes (0: no limit); returns
         what they hold now."""
         return _check(lib().gd_test_memory_limit(self.h, int(limit)))
+
+    def test_ahead(self, groups=0, seeds=0, traces=0):
+        """Test hook: capacities of the seeds aligned ahead (0: the defaults); returns the seeds
+        (listed, aligned ahead, taken) since the last call."""
+        n = (C.c_int64 * 3)()
+        _check(lib().gd_test_ahead(self.h, int(groups), int(seeds), int(traces), n))
+        return tuple(n)
 
     def las_merge(self, in_paths, out_path):
         """LAmerge of .las files on the device; returns the number of records."""

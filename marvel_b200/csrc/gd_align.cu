@@ -3035,7 +3035,7 @@ __device__ __forceinline__ void panel_scores(const uint64_t* __restrict__ hkey, 
 template <int RG>
 __device__ __noinline__ bool take_ahead(WarpSmem<RG>* sm, uint16_t* pts, int ptscap, int lane,
                                         const AheadPath* __restrict__ path, int n, const uint16_t* __restrict__ trace,
-                                        int diag, int apos)
+                                        int diag, int apos, unsigned* taken)
 {
     for (int base = 0; base < n; base += 32)
     {
@@ -3051,6 +3051,7 @@ __device__ __noinline__ bool take_ahead(WarpSmem<RG>* sm, uint16_t* pts, int pts
             sm->ap = LAPath{p.abpos, p.bbpos, p.aepos, p.bepos, p.diffs, p.atlen, 0, 0};
             sm->bp = LAPath{p.b_abpos, p.b_bbpos, p.b_aepos, p.b_bepos, p.diffs, p.btlen, p.atlen, 0};
             sm->wv_cells = p.cells;
+            atomicAdd(taken, 1u);
         }
         for (int k = lane; k < p.atlen + p.btlen; k += 32)
             pts[k] = trace[p.at + k];
@@ -3274,7 +3275,7 @@ __global__ void __launch_bounds__(warps_of<RG>() * 32, RG == WIDE_RING ? 1 : GD_
                     nseeds++;
                     int bpj = apj - dj;
                     if (AHEAD && ahead.y && take_ahead<RG>(w.sm, w.pts, w.ptscap, lane, out.ahead.path + ahead.x,
-                                                           (int)ahead.y, out.ahead.trace, dj, apj))
+                                                           (int)ahead.y, out.ahead.trace, dj, apj, out.ahead.ctr + 3))
                         w.cells += w.sm->wv_cells;
                     else
                         local_alignment<RG, true>(w, P, aseq, bseq, A.pk, ag, B.pk, bg, alen, blen, P.comp, dj,
@@ -4193,8 +4194,8 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32)
     if (lane == 0)
         first = atomicAdd(&ah.ctr[0], n);
     first = __shfl_sync(GD_FULL, first, 0);
-    const bool room = first + n <= (unsigned)AHEAD_CAP;
-    for (unsigned t = lane; t < n && first + t < (unsigned)AHEAD_CAP; t += 32)
+    const bool room = first + n <= ah.room;
+    for (unsigned t = lane; t < n && first + t < ah.room; t += 32)
     {
         AheadPath& p = ah.path[first + t];
         p.item = room ? (int)item : -1;
@@ -4225,7 +4226,7 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32, GD_ALIGN_MINB)
     w.ptscap = sc.ptscap;
     w.st = st;
     w.lane = lane;
-    const unsigned total = min(ah.ctr[0], (unsigned)AHEAD_CAP);
+    const unsigned total = min(ah.ctr[0], ah.room);
     while (true)
     {
         unsigned q = 0;
@@ -4263,8 +4264,11 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32, GD_ALIGN_MINB)
         for (int i = lane; i < b.tlen; i += 32)
             ah.trace[t0 + a.tlen + i] = w.pts[b.toff + i];
         if (lane == 0)
+        {
             *out = AheadPath{item,    diag,    apos,    1,       a.abpos, a.bbpos, a.aepos, a.bepos, a.diffs,
                              a.tlen,  b.abpos, b.bbpos, b.aepos, b.bepos, b.tlen,  w.cells, t0};
+            atomicAdd(&ah.ctr[2], 1u);
+        }
         __syncwarp();
     }
 }
@@ -4273,7 +4277,7 @@ int launch_align_ahead(const DevBlock& A, const DevBlock& B, const uint64_t* hke
                        const uint2* groups, const uint32_t* order, unsigned nheavy, const uint8_t* skip, AlignParams p,
                        AlignScratch sc, Ahead ah, DevStatus* st, int grid, cudaStream_t s, bool* any)
 {
-    GD_CUDA(cudaMemsetAsync(ah.groups, 0, AHEAD_GROUPS * sizeof(uint2) + 16, s));  // ctr and top follow groups
+    GD_CUDA(cudaMemsetAsync(ah.groups, 0, AHEAD_GROUPS * sizeof(uint2) + 24, s));  // ctr and top follow groups
     const unsigned n = nheavy < (unsigned)AHEAD_GROUPS ? nheavy : (unsigned)AHEAD_GROUPS;
     k_ahead_seeds<<<(n + ALIGN_WARPS - 1) / ALIGN_WARPS, ALIGN_WARPS * 32, 0, s>>>(hkey, hdiag, groups, order, n, skip, p,
                                                                                   sc, ah);

@@ -102,11 +102,12 @@ struct AheadPath
 struct Ahead
 {
     uint2* groups;      // (first, count) of a group's seeds in path [AHEAD_GROUPS]; null: none are aligned ahead
-    AheadPath* path;    // [AHEAD_CAP]
-    unsigned* ctr;      // [0] seeds, [1] queue; right behind groups, top behind them
+    AheadPath* path;    // [room]
+    unsigned* ctr;      // [0] seeds, [1] queue, [2] aligned, [3] taken; right behind groups, top behind them
     unsigned long long* top;  // trace values used
     uint16_t* trace;
-    unsigned long long cap;
+    unsigned long long cap;  // of trace
+    unsigned room;      // of path, AHEAD_CAP but in tests
 };
 
 struct AlignOut

@@ -161,6 +161,9 @@ int bits_for(int64_t maxval)
 
 }  // namespace
 
+// trace values of the seeds aligned ahead of one orientation (a seed without room is left to the aligner)
+constexpr size_t AHEAD_TRACE = 48u << 20;
+
 struct gd_context
 {
     // calls from several threads take turns: buffers, staging and scratch outlive a call and are
@@ -192,6 +195,10 @@ struct gd_context
     DevBuf ascr_d;        // the duo instance's scratch
     DevBuf ah_path, ah_misc, ah_trace;  // seeds aligned ahead of the aligner
     int agrid_d = 0;
+    // tests: smaller capacities of theirs, and how many seeds were listed, aligned and taken
+    unsigned ah_groups = gd::AHEAD_GROUPS, ah_seeds = gd::AHEAD_CAP;
+    size_t ah_traces = AHEAD_TRACE;
+    int64_t ah_count[3] = {};
     int test_narrow = 0;  // tests only: the main aligner pass with the 32-diagonal instance
     // aligner schedule: empty = every pair group in one persistent launch (longest first from
     // the device queue); else one launch per length class, split at these alen + blen edges
@@ -1003,9 +1010,6 @@ static int match_filter_d2_t(gd_context* c, int bslot, int cslot, int self)
     return 0;
 }
 
-// trace values of the seeds aligned ahead of one orientation (a seed without room is left to the aligner)
-constexpr size_t AHEAD_TRACE = 48u << 20;
-
 // The hits of one orientation in (hk0, hd0), in generation order, through the hit sort, the
 // pair groups, the learned triage and the seed scan + alignment; records are appended to the
 // overlap buffer in HBM.  c->ev0 marks the start of this orientation's merge stage.
@@ -1250,7 +1254,7 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
         c->kept_ah.busy = true;
         const bool ahead = nheavy && !ensure(c->ah_path, AHEAD_CAP * sizeof(AheadPath)) &&
                            !ensure(c->ah_trace, AHEAD_TRACE * 2) &&
-                           !ensure(c->ah_misc, AHEAD_GROUPS * sizeof(uint2) + 16 + sizeof(DevStatus));
+                           !ensure(c->ah_misc, AHEAD_GROUPS * sizeof(uint2) + 24 + sizeof(DevStatus));
         if (nheavy && !ahead)
             for (DevBuf* b : c->kept_ah.bufs)
                 dev_free(*b);
@@ -1258,14 +1262,16 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
         {
             bool any = false;
             Ahead ah{};
-            ah.cap = AHEAD_TRACE;
+            ah.cap = c->ah_traces;
+            ah.room = c->ah_seeds;
             ah.path = P<AheadPath>(c->ah_path);
             ah.trace = P<uint16_t>(c->ah_trace);
             ah.groups = P<uint2>(c->ah_misc);
             ah.ctr = (unsigned*)(ah.groups + AHEAD_GROUPS);
-            ah.top = (unsigned long long*)(ah.ctr + 2);
-            if (launch_align_ahead(A.blk, B.blk, hkey, hdiag, P<uint2>(c->groups), order, nheavy, skip, ap, ks[0], ah,
-                                   (DevStatus*)(ah.ctr + 4), kgrid[0], s, &any))
+            ah.top = (unsigned long long*)(ah.ctr + 4);
+            if (launch_align_ahead(A.blk, B.blk, hkey, hdiag, P<uint2>(c->groups), order,
+                                   std::min(nheavy, c->ah_groups), skip, ap, ks[0], ah, (DevStatus*)(ah.top + 1),
+                                   kgrid[0], s, &any))
                 return -1;
             if (any)
                 out.ahead = ah;
@@ -1286,8 +1292,10 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
         }
         // pair groups whose band outgrew the main instance: the wide one, appending to the same
         // output with its own scratch (a band wider than WIDE_RING is an error there)
-        unsigned nwide = 0;
+        unsigned nwide = 0, ahc[4] = {};
         GD_CUDA(cudaMemcpyAsync(&nwide, d_nwide, 4, cudaMemcpyDeviceToHost, s));
+        if (out.ahead.groups)
+            GD_CUDA(cudaMemcpyAsync(ahc, out.ahead.ctr, sizeof ahc, cudaMemcpyDeviceToHost, s));
         GD_CUDA(cudaStreamSynchronize(s));
         c->kept_ah.busy = false;  // the seeds are taken: what follows may have the memory
         c->stats.wide[oi] = nwide;
@@ -1317,6 +1325,8 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
         unsigned long long cnt[8];
         GD_CUDA(cudaMemcpy(&st, c->status.p, sizeof(st), cudaMemcpyDeviceToHost));
         GD_CUDA(cudaMemcpy(cnt, c->counters.p, sizeof(cnt), cudaMemcpyDeviceToHost));
+        for (int i = 0; i < 3; i++)
+            c->ah_count[i] += ahc[i ? i + 1 : 0];
         if (st.code != 0)
         {
             if (st.code == GD_ERR_PEBBLES)
@@ -2616,6 +2626,21 @@ int gd_test_wait_expiry(gd_context* c, int polls)
     if (gd::radix_sort_test_wait_expiry(polls, c->s))
         return -2;
     return gd::radix_sort_wait_check(c->s);
+}
+
+int gd_test_ahead(gd_context* c, int64_t groups, int64_t seeds, int64_t traces, int64_t counts[3])
+{
+    Turn turn(c);
+    auto cap = [](int64_t v, int64_t most) { return v > 0 && v < most ? v : most; };
+    c->ah_groups = (unsigned)cap(groups, gd::AHEAD_GROUPS);
+    c->ah_seeds = (unsigned)cap(seeds, gd::AHEAD_CAP);
+    c->ah_traces = (size_t)cap(traces, (int64_t)AHEAD_TRACE);
+    for (int i = 0; i < 3; i++)
+    {
+        counts[i] = c->ah_count[i];
+        c->ah_count[i] = 0;
+    }
+    return 0;
 }
 
 int64_t gd_test_memory_limit(gd_context* c, int64_t bytes)
