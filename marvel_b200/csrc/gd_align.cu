@@ -3262,16 +3262,20 @@ __global__ void __launch_bounds__(warps_of<RG>() * 32, RG == WIDE_RING ? 1 : GD_
                     int sc0 = score[dg];
                     cand = (sc0 + score[dg + 1] >= P.hitmin) || (sc0 + score[dg - 1] >= P.hitmin);
                 }
-                unsigned cm = __ballot_sync(GD_FULL, cand);
-                while (cm && !w.err && !pb.err)
+                // the lanes look at their bands' lasta together, again after each alignment, which
+                // moves it: taken one by one, the thousands of candidates of an overlap of accurate
+                // reads, all but the first covered, cost as much as its alignment
+                unsigned rest = GD_FULL;
+                while (!w.err && !pb.err)
                 {
+                    const unsigned cm = __ballot_sync(GD_FULL, cand && ap > lasta[dg]) & rest;
+                    if (!cm)
+                        break;
                     int j = __ffs(cm) - 1;
-                    cm &= cm - 1;
+                    rest = ~1u << j;
                     int apj = __shfl_sync(GD_FULL, ap, j);
                     int dj = __shfl_sync(GD_FULL, d, j);
                     int dgj = dj >> BS;
-                    if (!(apj > lasta[dgj]))
-                        continue;
                     nseeds++;
                     int bpj = apj - dj;
                     if (AHEAD && ahead.y && take_ahead<RG>(w.sm, w.pts, w.ptscap, lane, out.ahead.path + ahead.x,
