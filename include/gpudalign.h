@@ -197,8 +197,9 @@ int64_t gd_test_memory_limit(gd_context* ctx, int64_t bytes);
 
 /* Test hook: the capacities (at most the defaults; 0: those) with which later comparisons align the
  * likely seeds of repeat groups ahead -- groups looked at, seeds, trace values -- and how many
- * seeds were listed, aligned ahead and taken by the pair kernel since the last call. */
-int gd_test_ahead(gd_context* ctx, int64_t groups, int64_t seeds, int64_t traces, int64_t counts[3]);
+ * seeds were listed, aligned ahead and taken by the pair kernel since the last call, and how many
+ * groups were looked for them. */
+int gd_test_ahead(gd_context* ctx, int64_t groups, int64_t seeds, int64_t traces, int64_t counts[4]);
 
 /* LAsort (dalign/LAsort.c:65-90, 139-256) of one .las file on the device: writes out_path
  * with the records of in_path ordered by (aread, bread, abpos) -- ties, which the

@@ -377,8 +377,8 @@ class Context:
 
     def test_ahead(self, groups=0, seeds=0, traces=0):
         """Test hook: capacities of the seeds aligned ahead (0: the defaults); returns the seeds
-        (listed, aligned ahead, taken) since the last call."""
-        n = (C.c_int64 * 3)()
+        (listed, aligned ahead, taken) since the last call, and the groups looked at."""
+        n = (C.c_int64 * 4)()
         _check(lib().gd_test_ahead(self.h, int(groups), int(seeds), int(traces), n))
         return tuple(n)
 

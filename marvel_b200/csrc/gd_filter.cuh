@@ -140,8 +140,8 @@ int launch_hit_unpack(const uint64_t* packed, int64_t n, HitBits hb, uint64_t* h
 // candidate seed in it (group_can_fire): such a group fires no Local_Alignment and yields
 // nothing, the scan would only have read its hits.  hitmin = 0 keeps every group with >=
 // minhit hits.  The order's cost is alen + blen, with byhits at least 16 times the group's hits (see
-// k_select_groups); groups of at least heavy hits, and of a hit per 32 bases of
-// alen + blen, come before all others (heavy 0: none do).  ngroups[0] counts the groups kept,
+// k_select_groups); groups of at least heavy hits, of a hit per 32 bases of alen + blen and on
+// many bands come before all others (heavy 0: none do).  ngroups[0] counts the groups kept,
 // ngroups[1] those.
 int launch_pair_flags(const uint64_t* hkey, int64_t n, int pbits, uint32_t* flags, cudaStream_t s);
 int launch_pair_scatter(const uint32_t* flags, const uint32_t* pos, int64_t n, uint32_t* starts, cudaStream_t s);

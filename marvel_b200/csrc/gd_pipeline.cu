@@ -195,10 +195,11 @@ struct gd_context
     DevBuf ascr_d;        // the duo instance's scratch
     DevBuf ah_path, ah_misc, ah_trace;  // seeds aligned ahead of the aligner
     int agrid_d = 0;
-    // tests: smaller capacities of theirs, and how many seeds were listed, aligned and taken
+    // tests: smaller capacities of theirs, and how many seeds were listed, aligned and
+    // taken of how many groups looked at
     unsigned ah_groups = gd::AHEAD_GROUPS, ah_seeds = gd::AHEAD_CAP;
     size_t ah_traces = AHEAD_TRACE;
-    int64_t ah_count[3] = {};
+    int64_t ah_count[4] = {};
     int test_narrow = 0;  // tests only: the main aligner pass with the 32-diagonal instance
     // aligner schedule: empty = every pair group in one persistent launch (longest first from
     // the device queue); else one launch per length class, split at these alen + blen edges
@@ -1327,6 +1328,7 @@ static int align_hits(gd_context* c, Slot& A, Slot& B, uint64_t nhits, gd::HitBi
         GD_CUDA(cudaMemcpy(cnt, c->counters.p, sizeof(cnt), cudaMemcpyDeviceToHost));
         for (int i = 0; i < 3; i++)
             c->ah_count[i] += ahc[i ? i + 1 : 0];
+        c->ah_count[3] += nheavy;
         if (st.code != 0)
         {
             if (st.code == GD_ERR_PEBBLES)
@@ -2628,14 +2630,14 @@ int gd_test_wait_expiry(gd_context* c, int polls)
     return gd::radix_sort_wait_check(c->s);
 }
 
-int gd_test_ahead(gd_context* c, int64_t groups, int64_t seeds, int64_t traces, int64_t counts[3])
+int gd_test_ahead(gd_context* c, int64_t groups, int64_t seeds, int64_t traces, int64_t counts[4])
 {
     Turn turn(c);
     auto cap = [](int64_t v, int64_t most) { return v > 0 && v < most ? v : most; };
     c->ah_groups = (unsigned)cap(groups, gd::AHEAD_GROUPS);
     c->ah_seeds = (unsigned)cap(seeds, gd::AHEAD_CAP);
     c->ah_traces = (size_t)cap(traces, (int64_t)AHEAD_TRACE);
-    for (int i = 0; i < 3; i++)
+    for (int i = 0; i < 4; i++)
     {
         counts[i] = c->ah_count[i];
         c->ah_count[i] = 0;
