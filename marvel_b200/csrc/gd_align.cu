@@ -4308,8 +4308,10 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32)
     k_la_batch(const uint32_t* apk, uint32_t apk0, const uint32_t* bpk, uint32_t bpk0, const uint8_t* abase, const int64_t* aoff, const int32_t* alen, const uint8_t* bbase,
                const int64_t* boff, const int32_t* blen, const int32_t* diag, const int32_t* anti, int nseeds,
                AlignParams P, AlignScratch sc, int32_t* out12, uint16_t* tr, int trstride, int64_t* cells,
-               DevStatus* st)
+               DevStatus* st, const unsigned* odd)
 {
+    if (odd && (*odd != 0) == PK)
+        return;  // the other instance's batch
     __shared__ WarpSmem<RING> smem[ALIGN_WARPS];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -4375,31 +4377,10 @@ __global__ void __launch_bounds__(ALIGN_WARPS * 32)
     }
 }
 
-// One of a seed's two reads: bases 0 to 3 between 4s.  16 bytes a lane, so that a warp takes a read of
-// 10 kbp in 20 loads (the reads lie in their buffers, which have a margin of 4s).
+// One of a seed's two reads: bases 0 to 3 between 4s
 __device__ __forceinline__ bool plain_read(const uint8_t* base, int64_t off, int32_t len, int lane)
 {
-    if (base[off - 1] != 4 || base[off + len] != 4)
-        return false;
-    const int64_t end = off + len;
-    bool ok = true;
-    for (int64_t i = (off & ~15ll) + 16 * lane; i < end; i += 512)
-    {
-        const uint4 v = *reinterpret_cast<const uint4*>(base + i);
-        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-        {
-            const int64_t lo = off - (i + 4 * j), hi = end - (i + 4 * j);  // the read's bytes of this word: [lo, hi)
-            uint32_t m = 0xfcfcfcfcu;
-            if (lo > 0)
-                m = lo < 4 ? m << (8 * lo) : 0u;
-            if (hi < 4)
-                m &= hi > 0 ? 0xffffffffu >> (8 * (4 - hi)) : 0u;
-            ok = ok && (q[j] & m) == 0;
-        }
-    }
-    return ok;
+    return base[off - 1] == 4 && base[off + len] == 4 && plain_bases(base + off, len, lane, 32);
 }
 
 // *odd = 1 when a seed's read is not as blocks hold it; a warp per seed
@@ -4429,7 +4410,7 @@ int launch_la_batch(const uint8_t* aseq_base, const int64_t* aoff, const int32_t
                     const int64_t* boff, const int32_t* blen, const int32_t* diag, const int32_t* anti, int nseeds,
                     AlignParams p, AlignScratch sc, int32_t* out12, uint16_t* tr, int trstride, int64_t* cells,
                     DevStatus* st, cudaStream_t s, const uint32_t* apk, uint32_t apk0, const uint32_t* bpk,
-                    uint32_t bpk0)
+                    uint32_t bpk0, const unsigned* odd)
 {
     if (nseeds <= 0)
         return 0;
@@ -4437,12 +4418,12 @@ int launch_la_batch(const uint8_t* aseq_base, const int64_t* aoff, const int32_t
     if (apk)
         k_la_batch<true><<<grid, ALIGN_WARPS * 32, 0, s>>>(apk, apk0, bpk, bpk0, aseq_base, aoff, alen, bseq_base, boff,
                                                            blen, diag, anti, nseeds, p, sc, out12, tr, trstride, cells,
-                                                           st);
-    else
+                                                           st, odd);
+    if (!apk || odd)
         k_la_batch<false><<<grid, ALIGN_WARPS * 32, 0, s>>>(nullptr, 0, nullptr, 0, aseq_base, aoff, alen, bseq_base,
                                                             boff, blen, diag, anti, nseeds, p, sc, out12, tr, trstride,
-                                                            cells, st);
-    GD_LAUNCHED(1);
+                                                            cells, st, odd);
+    GD_LAUNCHED(apk && odd ? 2 : 1);
     GD_CUDA(cudaGetLastError());
     return 0;
 }

@@ -154,12 +154,13 @@ int launch_la_plain(const uint8_t* aseq_base, const int64_t* aoff, const int32_t
 // One Local_Alignment per seed (for parity tests of the wave alone).  out12 per seed:
 // A-path {abpos,bbpos,aepos,bepos,diffs,tlen}, B-path the same; traces at
 // tr + seed * trstride (A) and tr + seed * trstride + trstride/2 (B).  With the buffers' 2-bit copies
-// (apk, bpk; byte 0 of the buffers at index apk0, bpk0) the waves read those.
+// (apk, bpk; byte 0 of the buffers at index apk0, bpk0) the waves read those, unless *odd, which
+// launch_la_plain sets on the same stream, is not 0: then the bytes.
 int launch_la_batch(const uint8_t* aseq_base, const int64_t* aoff, const int32_t* alen, const uint8_t* bseq_base,
                     const int64_t* boff, const int32_t* blen, const int32_t* diag, const int32_t* anti, int nseeds,
                     AlignParams p, AlignScratch sc, int32_t* out12, uint16_t* tr, int trstride, int64_t* cells,
                     DevStatus* st, cudaStream_t s, const uint32_t* apk = nullptr, uint32_t apk0 = 0,
-                    const uint32_t* bpk = nullptr, uint32_t bpk0 = 0);
+                    const uint32_t* bpk = nullptr, uint32_t bpk0 = 0, const unsigned* odd = nullptr);
 
 // Test hook: daligner2's Handle_Redundancies of one pair on one device thread (see gd_align.cu).
 int launch_test_hr_d2(const uint8_t* aseq, const uint8_t* bseq, int alen, int blen, int tspace, int comp, int novls,

@@ -101,6 +101,31 @@ __device__ __forceinline__ void gd_fail(DevStatus* st, int code, int where, int 
     }
 }
 
+// Whether p[0 .. len) holds bytes 0 to 3 only, as far as thread t of n looks: 16 bytes a thread and step
+// (10 kbp in 20 steps of a warp).  Up to 15 bytes before and behind are read too.
+__device__ __forceinline__ bool plain_bases(const uint8_t* p, int len, int t, int n)
+{
+    const int skew = (int)((uintptr_t)p & 15);
+    bool ok = true;
+    for (int64_t i = 16ll * t - skew; i < len; i += 16ll * n)
+    {
+        const uint4 v = *reinterpret_cast<const uint4*>(p + i);
+        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            const int64_t lo = -(i + 4 * j), hi = len - (i + 4 * j);  // the bytes of this word: [lo, hi)
+            uint32_t m = 0xfcfcfcfcu;
+            if (lo > 0)
+                m = lo < 4 ? m << (8 * lo) : 0u;
+            if (hi < 4)
+                m &= hi > 0 ? 0xffffffffu >> (8 * (4 - hi)) : 0u;
+            ok = ok && (q[j] & m) == 0;
+        }
+    }
+    return ok;
+}
+
 __device__ __forceinline__ unsigned lanemask_lt()
 {
     unsigned m;

@@ -145,7 +145,8 @@ struct Slot
     int64_t totlen = 0, nslots = 0;
     int64_t nmask = 0;  // ints of mask interval data
     int has_mask = 0, loaded = 0;
-    int plain = -1;  // reads of bases 0 to 3 only; -1: not looked at yet
+    DevBuf odd;       // a word: not 0 when a read holds a byte beyond 3, which the 2-bit copy loses,
+    int looked = 0;   // once the block has been looked at
     DevBuf code, read, rpos;
     int64_t nk = -1;
     std::vector<int32_t> hrlen;
@@ -1743,7 +1744,7 @@ int gd_load_block(gd_context* c, int slot, const gd_block* b)
     s.nslots = nb - (int64_t)c->kmer * b->nreads;
     s.hrlen.assign(b->rlen, b->rlen + b->nreads);
     s.loaded = 1;
-    s.plain = -1;
+    s.looked = 0;
     s.nk = -1;
     GD_CUDA(cudaStreamSynchronize(c->s));
     return 0;
@@ -1810,7 +1811,7 @@ int gd_complement_block(gd_context* c, int src, int dst)
     D.nslots = S.nslots;
     D.hrlen = S.hrlen;
     D.loaded = 1;
-    D.plain = S.plain;
+    D.looked = 0;
     D.nk = -1;
     GD_CUDA(cudaStreamSynchronize(c->s));
     return 0;
@@ -2403,29 +2404,20 @@ int gd_write_overlap_buffer(gd_context* c, int run_id, const char* ablock, const
     return write_las(c, p2, j, nsrt);
 }
 
-// whether all bases of the slots' blocks are 0 to 3 (the 2-bit copies hold no others): 1, 0, or -1 on failure
-static int slots_plain(gd_context* c, std::initializer_list<Slot*> slots)
+// the slots' odd words, on the context's stream
+static int look_at_slots(gd_context* c, std::initializer_list<Slot*> slots)
 {
-    unsigned odd[3], n = 0;
-    Slot* unknown[3];
-    if (ensure(c->vf_misc, 64))
-        return -1;
-    GD_CUDA(cudaMemsetAsync(c->vf_misc.p, 0, sizeof odd, c->s));
     for (Slot* s : slots)
-        if (s->loaded && s->plain < 0 && std::find(unknown, unknown + n, s) == unknown + n)
+        if (s->loaded && !s->looked)
         {
-            if (gd::launch_block_plain(s->blk, P<unsigned>(c->vf_misc) + n, c->s))
+            if (ensure(s->odd, 4))
                 return -1;
-            unknown[n++] = s;
+            GD_CUDA(cudaMemsetAsync(s->odd.p, 0, 4, c->s));
+            if (gd::launch_block_plain(s->blk, P<unsigned>(s->odd), c->s))
+                return -1;
+            s->looked = 1;
         }
-    if (n)
-    {
-        GD_CUDA(cudaMemcpyAsync(odd, c->vf_misc.p, sizeof odd, cudaMemcpyDeviceToHost, c->s));
-        GD_CUDA(cudaStreamSynchronize(c->s));
-    }
-    for (unsigned i = 0; i < n; i++)
-        unknown[i]->plain = !odd[i];
-    return std::all_of(slots.begin(), slots.end(), [](Slot* s) { return !s->loaded || s->plain; });
+    return 0;
 }
 
 int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const gd_overlap* recs, const uint8_t* trace,
@@ -2514,9 +2506,9 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
     const DevBlock& Cb = Cc.loaded ? Cc.blk : B.blk;
     cudaStream_t s = c->s;
     InUse use(c->kept_vf, KEPT_BYTES);
-    const int plain = slots_plain(c, {&A, &B, &Cc});
-    if (plain < 0)
+    if (look_at_slots(c, {&A, &B, &Cc}))
         return -1;
+    const unsigned* const odd[3] = {P<unsigned>(A.odd), P<unsigned>(B.odd), P<unsigned>((Cc.loaded ? Cc : B).odd)};
     if (ensure(c->vf_rec, (size_t)n * sizeof(OutRec)) || ensure(c->vf_first, (size_t)(n + 1) * 8) ||
         ensure(c->vf_trace, (size_t)(thi - tlo) + 16) || ensure(c->vf_seg, (size_t)nseg * sizeof(Segment)) ||
         ensure(c->vf_list, (size_t)nseg * 4) || ensure(c->vf_diff, (size_t)n * 4) || ensure(c->vf_misc, 64))
@@ -2537,7 +2529,7 @@ int gd_compute_trace_pts(gd_context* c, int aslot, int bslot, int cslot, const g
     if (launch_trace_segments(P<OutRec>(c->vf_rec), n, P<int64_t>(c->vf_first), P<uint8_t>(c->vf_trace), tlo, TS, tbytes,
                               A.blk.ufirst, B.blk.ufirst, P<Segment>(c->vf_seg), misc + 1, dst, s) ||
         launch_trace_pts(A.blk, B.blk, Cb, P<Segment>(c->vf_seg), nseg, P<int>(c->vf_diff), P<unsigned>(c->vf_list), misc,
-                         plain, s))
+                         odd, s))
         return -1;
     unsigned h[8];
     GD_CUDA(cudaMemcpyAsync(h, misc, sizeof h, cudaMemcpyDeviceToHost, s));
@@ -2732,6 +2724,9 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     DevStatus* d_st = P<DevStatus>(c->lb_out);
     int64_t* d_cells = (int64_t*)(P<char>(c->lb_out) + 64);
     int32_t* d_out = (int32_t*)(d_cells + nseeds);
+    GD_CUDA(cudaMemsetAsync(c->lb_out.p, 0, n8 + 12 * n4 + 64, s));
+    // the rows go to the caller whole: zeros behind a trace, not an earlier call's
+    GD_CUDA(cudaMemsetAsync(c->lb_tr.p, 0, (size_t)nseeds * trstride * 2, s));
     // sequences: caller buffers hold [4, read, 4, read, ...] with offsets relative to index 0
     GD_CUDA(cudaMemsetAsync(c->lb_a.p, 4, abytes, s));
     GD_CUDA(cudaMemsetAsync(c->lb_b.p, 4, bbytes, s));
@@ -2744,25 +2739,15 @@ int gd_local_alignment_batch(gd_context* c, const uint8_t* abases, int64_t alen_
     GD_CUDA(cudaMemcpyAsync(d_bl, blen, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_dg, diag, n4, cudaMemcpyHostToDevice, s));
     GD_CUDA(cudaMemcpyAsync(d_an, anti, n4, cudaMemcpyHostToDevice, s));
-    GD_CUDA(cudaMemsetAsync(c->lb_out.p, 0, n8 + 12 * n4 + 64, s));
-    // the rows go to the caller whole: zeros behind a trace, not an earlier call's
-    GD_CUDA(cudaMemsetAsync(c->lb_tr.p, 0, (size_t)nseeds * trstride * 2, s));
-    if (packed)
-    {
-        unsigned odd = 0, *d_odd = (unsigned*)(d_st + 1);
-        if (launch_la_plain(P<uint8_t>(c->lb_a) + LA_PAD, d_ao, d_al, P<uint8_t>(c->lb_b) + LA_PAD, d_bo, d_bl, nseeds,
-                            d_odd, s))
-            return -1;
-        GD_CUDA(cudaMemcpyAsync(&odd, d_odd, 4, cudaMemcpyDeviceToHost, s));
-        GD_CUDA(cudaStreamSynchronize(s));
-        packed = !odd;
-    }
-    if ((packed && (launch_pack2(P<uint8_t>(c->lb_a), abytes, P<uint32_t>(c->lb_pka), wa, s) ||
+    unsigned* const d_odd = (unsigned*)(d_st + 1);
+    if ((packed && (launch_la_plain(P<uint8_t>(c->lb_a) + LA_PAD, d_ao, d_al, P<uint8_t>(c->lb_b) + LA_PAD, d_bo, d_bl,
+                                    nseeds, d_odd, s) ||
+                    launch_pack2(P<uint8_t>(c->lb_a), abytes, P<uint32_t>(c->lb_pka), wa, s) ||
                     launch_pack2(P<uint8_t>(c->lb_b), bbytes, P<uint32_t>(c->lb_pkb), wb, s))) ||
         launch_la_batch(P<uint8_t>(c->lb_a) + LA_PAD, d_ao, d_al, P<uint8_t>(c->lb_b) + LA_PAD, d_bo, d_bl, d_dg, d_an,
                         nseeds, ap, sc, d_out, P<uint16_t>(c->lb_tr), trstride, d_cells, d_st, s,
                         packed ? P<uint32_t>(c->lb_pka) : nullptr, LA_PAD, packed ? P<uint32_t>(c->lb_pkb) : nullptr,
-                        LA_PAD))
+                        LA_PAD, packed ? d_odd : nullptr))
         return -1;
     DevStatus st;
     GD_CUDA(cudaMemcpyAsync(&st, d_st, sizeof st, cudaMemcpyDeviceToHost, s));

@@ -165,7 +165,9 @@ __global__ void __launch_bounds__(VT) k_trace_segments(const OutRec* __restrict_
 constexpr int VBAND = 64;
 
 __global__ void __launch_bounds__(VT) k_trace_pts(DevBlock A, DevBlock B, DevBlock C, const Segment* __restrict__ seg,
-                                                 int64_t nseg, int* diffs, unsigned* list, unsigned* nlist, bool plain)
+                                                 int64_t nseg, int* diffs, unsigned* list, unsigned* nlist, const unsigned* __restrict__ oddA,
+                                                 const unsigned* __restrict__ oddB,
+                                                 const unsigned* __restrict__ oddC)
 {
     __shared__ int band[VBAND][VT];
     const int64_t s = (int64_t)blockIdx.x * VT + threadIdx.x;
@@ -178,7 +180,7 @@ __global__ void __launch_bounds__(VT) k_trace_pts(DevBlock A, DevBlock B, DevBlo
     const uint32_t b0 = PK_BIAS + (uint32_t)bb.boff[g.bread] + (uint32_t)g.bb;
     int low = min(0, del), hgh = max(0, del), d = -1;
     const int room = (VBAND - (hgh - low + 3)) / 2;  // diagonals the band can grow on either side
-    if (plain && hgh - low + 3 <= VBAND && N < 32000)
+    if (!(*oddA | *oddB | *oddC) && hgh - low + 3 <= VBAND && N < 32000)
     {
         int* const w0 = &band[0][threadIdx.x] - (low - 1 - room) * VT;  // diagonal k at w0[k * VT]
         const int lo = low - 1 - room, hi = hgh + 1 + room;
@@ -268,12 +270,7 @@ __global__ void __launch_bounds__(VT) k_trace_pts_list(DevBlock A, DevBlock B, D
 // *odd = 1 when a read holds a byte beyond 3; a CTA per read
 __global__ void __launch_bounds__(VT) k_block_plain(DevBlock b, unsigned* odd)
 {
-    const uint8_t* s = b.bases + b.boff[blockIdx.x];
-    const int len = b.rlen[blockIdx.x];
-    unsigned any = 0;
-    for (int p = threadIdx.x; p < len; p += VT)
-        any |= s[p];
-    if (any > 3)
+    if (!plain_bases(b.bases + b.boff[blockIdx.x], b.rlen[blockIdx.x], threadIdx.x, VT))
         *odd = 1;
 }
 
@@ -301,7 +298,7 @@ int launch_trace_segments(const OutRec* recs, int64_t n, const int64_t* first, c
 }
 
 int launch_trace_pts(const DevBlock& A, const DevBlock& B, const DevBlock& C, const Segment* seg, int64_t nseg,
-                     int* diffs, unsigned* list, unsigned* nlist, bool plain, cudaStream_t s)
+                     int* diffs, unsigned* list, unsigned* nlist, const unsigned* const odd[3], cudaStream_t s)
 {
     if (nseg <= 0)
         return 0;
@@ -310,7 +307,7 @@ int launch_trace_pts(const DevBlock& A, const DevBlock& B, const DevBlock& C, co
         gd_set_error("%lld trace segments exceed the 32-bit segment index of this build", (long long)nseg);
         return -1;
     }
-    k_trace_pts<<<(unsigned)((nseg + VT - 1) / VT), VT, 0, s>>>(A, B, C, seg, nseg, diffs, list, nlist, plain);
+    k_trace_pts<<<(unsigned)((nseg + VT - 1) / VT), VT, 0, s>>>(A, B, C, seg, nseg, diffs, list, nlist, odd[0], odd[1], odd[2]);
     GD_LAUNCHED(1);
     GD_CUDA(cudaGetLastError());
     return 0;

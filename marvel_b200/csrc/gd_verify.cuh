@@ -32,10 +32,10 @@ int launch_trace_segments(const OutRec* recs, int64_t n, const int64_t* first, c
 int launch_block_plain(const DevBlock& b, unsigned* odd, cudaStream_t s);
 
 // The distance of every segment added to its record's diffs; the segments that outgrow the
-// kernel's bands, and all of them where the blocks are not plain, are listed (*nlist preset 0) for
-// launch_trace_pts_list, which compares bytes.
+// kernel's bands, and all of them where a block's *odd (A's, B's, C's, on the device) is not 0, are
+// listed (*nlist preset 0) for launch_trace_pts_list, which compares bytes.
 int launch_trace_pts(const DevBlock& A, const DevBlock& B, const DevBlock& C, const Segment* seg, int64_t nseg,
-                     int* diffs, unsigned* list, unsigned* nlist, bool plain, cudaStream_t s);
+                     int* diffs, unsigned* list, unsigned* nlist, const unsigned* const odd[3], cudaStream_t s);
 
 // The listed segments with bands of any width: threads need 3 * (2R + 1) ints of scratch each,
 // R >= segment M + N + 4.
