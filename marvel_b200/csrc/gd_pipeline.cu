@@ -1713,6 +1713,8 @@ int gd_load_block(gd_context* c, int slot, const gd_block* b)
                 return -1;
             }
         }
+    s.loaded = 0;  // until all of it is there: its old buffers may be gone
+    s.nk = -1;
     if (ensure(s.bases, nb + 1 + 64) || ensure(s.boff, (b->nreads + 1) * 8) || ensure(s.rlen, b->nreads * 4 + 4))
         return -1;
     GD_CUDA(cudaMemsetAsync(s.bases.p, 4, nb + 1 + 64, c->s));
@@ -1781,6 +1783,8 @@ int gd_complement_block(gd_context* c, int src, int dst)
     std::vector<int64_t> boff_last(1);
     GD_CUDA(cudaMemcpy(boff_last.data(), S.blk.boff + n, 8, cudaMemcpyDeviceToHost));
     nb = boff_last[0];
+    D.loaded = 0;
+    D.nk = -1;
     if (ensure(D.bases, nb + 1 + 64) || ensure(D.boff, (n + 1) * 8) || ensure(D.rlen, n * 4 + 4))
         return -1;
     GD_CUDA(cudaMemsetAsync(D.bases.p, 4, nb + 1 + 64, c->s));

@@ -144,3 +144,31 @@ def test_comparison_without_room_for_seeds_ahead():
             assert got[0].tobytes() == want[0].tobytes() and got[1].tobytes() == want[1].tobytes()
         assert ctx.test_memory_limit() <= need - short
         ctx.close()
+
+
+def test_failed_load_leaves_the_slot_empty():
+    """A block, or a complement, that finds no memory: calls on its slot are errors until one is loaded."""
+    import marvel_b200 as mb
+    small, big = one_read(20000), one_read(40 << 20)
+    ctx = mb.Context()
+    ctx.set_filter_params()
+    ctx.new_align_spec(0.70, 100, small.freq)
+    for slot in (0, 2):
+        ctx.load_block(slot, small)
+        ctx.sort_kmers(slot)
+    ctx.load_block(1, big)
+    ctx.test_memory_limit(ctx.test_memory_limit() + (1 << 20))
+    with pytest.raises(mb.GpuError, match="cudaMalloc"):
+        ctx.load_block(0, big)
+    with pytest.raises(mb.GpuError, match="cudaMalloc"):
+        ctx.complement_block(1, 2)
+    for slot in (0, 2):
+        with pytest.raises(mb.GpuError, match="not loaded"):
+            ctx.sort_kmers(slot)
+        with pytest.raises(mb.GpuError, match="not loaded"):
+            ctx.dust(slot, small.freq)
+    with pytest.raises(mb.GpuError, match="built before"):
+        ctx.match_filter(1, 0, 0)
+    ctx.load_block(0, small)
+    assert ctx.sort_kmers(0) == 20000 - 13
+    ctx.close()
