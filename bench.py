@@ -73,7 +73,7 @@ def path_name():
 CACHE = os.environ.get("MARVEL_B200_CACHE", os.path.join(tempfile.gettempdir(), "marvel_b200_bench"))
 # k_align_pairs DRAM bytes (read + write) per wave cell, from the ncu capture of the cfg1
 # N-orientation launch (profiles/k_align_pairs_cfg1.md): 85.0 MB over 282 M cells
-ALIGN_DRAM_BYTES_PER_CELL = 84.96e6 / 282.0e6
+ALIGN_DRAM_BYTES_PER_CELL = (77.66e6 + 111.95e6) / 275.8e6
 # k-mer index build DRAM bytes per k-mer (extraction + 4 LSD passes), from the ncu capture of
 # the cfg1 index (profiles/filter_kernels_cfg1.md): 1,731 MB over 21.08 M k-mers
 INDEX_DRAM_BYTES_PER_KMER = 1731.2e6 / 21082465
@@ -399,12 +399,12 @@ def run_gpu(args):
                          "peak": round(issue_peak, 2), "unit": "T int lane-ops/s",
                          "frac": round(achieved / issue_peak, 4),
                          "traffic": int(ALIGN_DRAM_BYTES_PER_CELL * cells / 2),
-                         "traffic_source": "bytes per launch: dram read+write per wave cell of the cfg1 ncu capture "
-                                           "(profiles/k_align_pairs_cfg1.md) x this launch's cells",
+                         "traffic_source": "bytes per launch: dram read+write per wave cell of the 21 Mbp ncu capture "
+                                           "(profiles/k_align_pairs_regs_21mbp.md) x this launch's cells",
                          "peak_source": "derived: 148 SM x 128 lanes/clk x median SM clock under load",
-                         "issue_slots_busy": 0.765,
+                         "issue_slots_busy": 0.773,
                          "issue_source": "smsp__issue_active of the 21 Mbp ncu capture (profiles/k_align_pairs_regs_21mbp.md): "
-                                         "the kernel issues on 76 % of cycles; a wave is ~11 diagonals wide, so a "
+                                         "the kernel issues on 77 % of cycles; a wave is ~11 diagonals wide, so a "
                                          "warp instruction carries about a third of a warp of cells"},
             "roofline_filter": {"bound": "hbm", "kernel": "k-mer index (extract + 4 LSD passes)",
                                 "achieved": round(idx_bytes / (idx_ms / 1e3) / 1e9, 1),

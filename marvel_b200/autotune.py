@@ -9,11 +9,12 @@ keeps the fastest:
   device queue, or one launch per length class (classes of alen + blen, split at quantiles
   of the block's pair lengths);
 * per length class, the kernel instance: a warp per alignment with 128-diagonal wave rings
-  (4 warps per CTA, 6 CTAs per SM; a group whose band outgrows 128 diagonals is redone by the
+  (4 warps per CTA, 7 CTAs per SM; a group whose band outgrows 128 diagonals is redone by the
   wide instance), the wide instance (512-diagonal rings, one warp per CTA), which takes such
   groups in one pass, or the duo instance (two 16-lane teams per warp, each on its own pair
   group with 128-diagonal rings), meant to keep twice the lanes busy on the narrow bands most
-  waves have (it measures slower on every workload: the ring pairs halve the resident warps).
+  waves have (it measures slower on every workload: its ring pairs halve the resident warps, and
+  its waves stay in the rings where the warp instance holds narrow ones in registers).
 
 Candidates are timed on the loaded blocks (the aligner's device time of both orientations,
 gd_stats.ms_align, best of `repeats` runs).  The radix sorts have no choice here: their

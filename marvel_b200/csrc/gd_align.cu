@@ -7,15 +7,15 @@
 // are built lane-parallel (match-any groups per diagonal band), candidate seeds are taken
 // in hit order, and each fired seed runs the O(ND) wave with lanes over diagonals: the
 // wave vectors V (furthest anti-diagonal), T (60-column match bit vector; its popcount
-// is the reference's M), HA/HB (pebble heads), NA/NB (next trace-point marks) live in two
-// per-warp shared-memory rings indexed by diagonal, one per wave parity: each wave reads
-// the previous wave for diagonals k-1, k, k+1 and writes the other ring, which is the
-// reference's in-place update order.  A band of at most 30 diagonals (most waves) is held in
+// is the reference's M), HA/HB (pebble heads), NA/NB (next trace-point marks) live in a
+// shared-memory ring per warp indexed by diagonal, which a wave updates in place, a chunk of 32
+// diagonals at a time: every lane reads the previous wave at k-1, k, k+1 before any writes, and
+// the diagonal that the next chunk still reads is saved (ChunkEdge).  A band of at most 30 diagonals (most waves) is held in
 // registers instead, a diagonal per lane, and updated by shuffles (wave_regs).  The reference's
 // sequential "c > besta" scan over diagonals becomes a warp prefix-max in scan order; its clip
 // bookkeeping becomes ballots.
 // Pebbles go to a per-warp global arena; the two trace-point chains are unwound by lane 0.
-// Match extension compares 4 bases per step with 32-bit XOR windows.
+// Match extension compares 16 bases per step over the 2-bit reads (4 over bytes).
 //
 // Instances by ring size: RING (128 diagonals, 4 warps per CTA) aligns every pair group; a
 // group whose band grows wider is abandoned there (nothing emitted, its counts dropped) and
@@ -310,7 +310,7 @@ __device__ __forceinline__ int snake_pk(const bool FWD, const uint32_t* __restri
 }
 
 // snake_pk out of line for the 0-wave: (y, bend | aend << 1).  The pair kernel's code is near the size
-// its instruction cache holds (in line, the 121 Mbp block's aligner took 185.5 ms instead of 183).
+// its instruction cache holds (in line, the 121 Mbp block's aligner takes 167 ms instead of 162).
 __device__ __noinline__ int2 snake_begin(const bool FWD, const uint32_t* __restrict__ apk, uint32_t ag,
                                          const uint32_t* __restrict__ bpk, uint32_t bg, int y, int k, int alen, int blen)
 {
@@ -956,8 +956,9 @@ __device__ __forceinline__ bool wave_step(const bool FWD, WarpCtx<RG>& w, WaveVa
 // carries per diagonal are never ahead of or behind that), which the predecessor's position
 // gives, and so no pebble is read back for its mark either.  On a 21 Mbp block (25 M waves per
 // orientation) the kernel issues 6.6 G warp instructions instead of 8.2 G and takes 7.9 ms
-// instead of 9.4; with the extension's first 16 bases in line and fewer branches 6.4 G and 7.6 ms.
-// It stays bound by issue (76 % of the slots) and the dependent chain of a wave.
+// instead of 9.4; with the extension's first 16 bases in line, fewer branches and the covered seed
+// candidates passed over together 6.3 G and 7.4 ms.  It stays bound by issue (77 % of the slots) and
+// the dependent chain of a wave.
 //
 // Runs waves until the wave loop ends (false; or an error in w.err) or the band or anything
 // unusual asks for wave_step (true; the state is then in the ring).
@@ -3149,11 +3150,12 @@ constexpr int warps_of()
 // D2: daligner2's report (dalign2/filter_reporter_cpu.c) -- its -H, its rule for the B-side
 // record of a read against itself, its Handle_Redundancies; a separate instance, so that
 // daligner's keeps its code layout.  AHEAD: some groups have seeds aligned ahead (an instance of its
-// own for the same reason: with the look-up in the plain one the 121 Mbp block took 188 ms
-// instead of 183).
+// own for the same reason: with the look-up in the plain one the 121 Mbp block takes 163.3 and
+// 164.2 ms instead of 162.0 and 163.5).
 #ifndef GD_ALIGN_MINB
-// CTAs per SM the warp instance is compiled for, with the waves in registers: 7 (72 registers) runs the
-// 121 Mbp block's aligner in 183 ms per orientation, 6 (80) in 199, 8 (64) in 186
+// CTAs per SM the warp instance is compiled for: 7 (72 registers) runs the 121 Mbp block's aligner in 162
+// ms per orientation and the 53 Mbp block pair's with tandem repeats in 62.0 and 64.4, 6 (80) in
+// 166, 61.7 and 63.7, 8 (64) in 158, 64.0 and 66.0
 #define GD_ALIGN_MINB 7
 #endif
 
@@ -4106,10 +4108,11 @@ int launch_align_pairs(const DevBlock& A, const DevBlock& B, const uint64_t* hke
 // alignment moves lasta, which decides the next.  In a group of two reads that share a tandem
 // repeat (thousands of hits, a hundred alignments) that chain outlasts everything else in the
 // block: a 53 Mbp block pair kept one warp busy for 100 ms where its whole work is worth 40 (aligned
-// ahead: 90 and 107 ms of aligner per orientation become 70 and 78).  But
+// ahead, 90 and 107 ms of aligner per orientation became 70 and 78; now 62 and 64).  But
 // lasta is 0 on a band no alignment has touched, so the first candidate of every band is a
 // likely seed: these are aligned here first, each on a warp of its own, and the pair kernel,
-// running the same scan as ever, takes a seed's result if it is there (four in five are).  Seeds
+// running the same scan as ever, takes a seed's result if it is there (nine in ten of these groups'
+// seeds are; of the seeds aligned ahead a little under half are taken).  Seeds
 // that turn out to be covered are work for nothing, so only groups with a large share of the
 // block's hits (the host's rule) and a candidate on many bands are treated so.
 // ------------------------------------------------------------------------------------------

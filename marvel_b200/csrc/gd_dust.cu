@@ -2,8 +2,8 @@
 //
 // The scan of one read is a sequential state machine (a window of triplet counts, a
 // left-trimmed run with its own counts, a short list of candidate intervals).  Its state
-// after position j follows from the last 2W bases alone, so k_dust_chunks cuts every read into
-// chunks and gives each a thread that starts 2W positions early (below).  With -b the sums are
+// after position j follows from bases near j, so k_dust_chunks cuts every read into chunks and
+// gives each a thread that starts W positions early (below).  With -b the sums are
 // doubles whose rounding carries the read's whole past, so k_dust_read scans one read per
 // thread.  Each read's mask is written to its own slice of a device buffer.  Arithmetic follows the
 // reference's types: integer pair-count sums, doubles for the thresholds, and with -b
@@ -194,13 +194,13 @@ __global__ void __launch_bounds__(64) k_dust_read(DevBlock blk, int W, double T,
 // candidate that starts at x is made, raised and tested at positions from x to x + W - 2 only, with
 // windows that reach back to x - W, against candidates that start at or behind x.  So a scan
 // begun W positions before the chunk, which makes candidates from the chunk's first start on
-// only, has the same candidates there as the whole read's scan.  The chunk's retired candidates come in order of their
-// starts and are merged as the reference merges them; k_dust_merge joins the chunks' lists,
-// which merges the same sequence in pieces.
+// only, has the same candidates there as the whole read's scan.  The chunk's retired candidates come
+// in order of their starts and are merged as the reference merges them; k_dust_merge joins the
+// chunks' lists, which merges the same sequence in pieces.
 //
 // One thread per read (a 105 Mbp block of 10,020 reads) took 91 ms, its longest reads deciding.
-// With chunks the bound is divergence: one step in ten or so walks the window from the run's start
-// down to its own (up to W - 2 places), and with the walk as an inner loop nearly every step of a
+// With chunks the bound is divergence: one step in twenty or so walks the window from the run's start
+// down to its own (up to W - 2 places, 29 on average), and with the walk as an inner loop nearly every step of a
 // warp waited for some lane's (20 ms at any chunk size).  So a lane is either stepping or walking,
 // and every turn of the one loop takes each lane one step or one place further.  The walk counts
 // the triplets it meets on top of the run's in a field of its own, valid under the walk's tag,
