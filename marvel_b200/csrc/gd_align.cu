@@ -1654,6 +1654,23 @@ __device__ __forceinline__ bool wave_step_duo(bool go, const bool FWD, WarpCtx<D
     return go;
 }
 
+// Byte waves end at 4s, which may stand behind a length, and then pass more trace points than the lengths
+// give room for (lane 0).  Room of A's and B's values around their first: A's forward ones run
+// towards B's reverse ones.
+template <int RG>
+__device__ bool trace_room(const bool fwd, const WarpCtx<RG>& w, int ha, int hb, int TS, int alen, int blen, int atlen)
+{
+    const int maxtp = 2 * (max(alen, blen) / TS + 2);
+    int need[2] = {0, 0};  // a pair of values per pebble at most, the last point in place of the first
+    for (int i = 0; i < 2; i++)
+        for (int h = i ? hb : ha; h >= 0; h = w.peb[h].x)
+            need[i] += 2;
+    if (fwd ? need[0] <= 2 * maxtp && need[1] <= w.ptscap - 3 * maxtp : need[0] <= maxtp && need[1] <= 2 * maxtp - atlen)
+        return true;
+    gd_fail(w.st, GD_ERR_TRACE, w.item, maxtp);
+    return false;
+}
+
 template <int RG, bool PK>
 __device__ __forceinline__ void wave_end(const bool FWD, WarpCtx<RG>& w, WaveVars& wvars, const AlignParams& P, const uint8_t* aseq0, const uint8_t* bseq0,
     const uint32_t* apk, uint32_t ag, const uint32_t* bpk, uint32_t bg, int alen, int blen, int comp, LAPath* apath, LAPath* bpath, int* mind, int mida,
@@ -1673,6 +1690,21 @@ __device__ __forceinline__ void wave_end(const bool FWD, WarpCtx<RG>& w, WaveVar
     int low = wvars.low;
     // ---- trace points of both paths from the pebble chains (align.c:970-1106, 1710-1902)
     tsync(w);
+    if constexpr (!PK)
+    {
+        if (lane == 0)
+        {
+            const bool clipped = clipm[0] >= 0;
+            w.sm->wv_err = !trace_room(FWD, w, clipped ? clipm[4] : trim[3], clipped ? clipm[5] : trim[4], TS, alen, blen,
+                                       apath->tlen);
+        }
+        tsync(w);
+        if (w.sm->wv_err)
+        {
+            w.err = 1;
+            return;
+        }
+    }
     if (lane == 0)
     {
         int4* cells = w.peb;

@@ -152,3 +152,26 @@ def test_results_do_not_depend_on_earlier_calls(ctx):
     half = got[1].shape[1] // 2
     for o, row in zip(*got[:2]):
         assert not row[o[5]:half].any() and not row[half + o[11]:].any()
+
+
+@pytest.mark.parametrize("comp", [0, 1])
+@pytest.mark.parametrize("length,fits", [(2999, True), (2500, True), (100, False)])
+def test_length_far_below_the_read(ctx, length, fits, comp):
+    """Byte waves run on to the read's 4, up to a match of the length at a time: where the trace outgrows
+    the room that the lengths give it, an error of that seed (code 3), and the context goes on."""
+    import marvel_b200 as mb
+    rng = np.random.default_rng(60 + comp)
+    s = rng.integers(0, 4, 3000, dtype=np.uint8)
+    t = s.copy()
+    t[80::90] = (t[80::90] + 1) & 3
+    abuf, aoff, alen = joined([s])
+    bbuf, boff, blen = joined([t])
+    n = np.array([length], np.int32)
+    for at in (0, min(length, 1400)):
+        call = (abuf, aoff, n, bbuf, boff, n, [0], [2 * at], comp)
+        out = same_as_bytes(ctx, *call)
+        assert (out is not None) == fits
+        if not fits:
+            with pytest.raises(mb.GpuError, match="code 3"):
+                ctx.local_alignment_batch(*call)
+    assert same_as_bytes(ctx, abuf, aoff, alen, bbuf, boff, blen, [0], [0], comp) is not None
